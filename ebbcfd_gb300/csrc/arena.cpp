@@ -568,6 +568,15 @@ int assemble(ebb_solver *s, std::vector<InstLayout> &Ls, int32_t precision, std:
     M.Eint = (int32_t)Et;
     M.maxJ = MJ;
     M.uniform = std::all_of(nedge.begin(), nedge.end(), [&](int32_t v) { return v == MJ; }) ? 1 : 0;
+    // what the FP64 kernels' integer-pipe products and FP32 limiter decisions assume
+    auto within = [](const std::vector<double> &v, double top) {
+        return std::all_of(v.begin(), v.end(), [top](double x) {
+            const double a = std::fabs(x);
+            return a == 0.0 || (a >= 0x1p-100 && a < top);
+        });
+    };
+    M.soft = precision == EBB_PREC_FP64 && within(sgm, 0x1p100) && within(snd, 0x1p20) && within(sfd, 0x1p20) &&
+             within(en, 2.0);
     M.n_inst = n;
     M.n_upd_blocks = nblk;
     auto up = [&](auto *dst, const auto &v) {

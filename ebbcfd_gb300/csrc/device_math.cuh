@@ -36,12 +36,11 @@ template <> struct K<df> {  // the double constants, as double-floats
     static constexpr df g = df(1.4), gm1 = df(1.4 - 1), gm1d = df(1.4 - 1.0);
 };
 
-// Quotients by one divisor.  FP64: one correctly rounded reciprocal of the divisor
-// serves every quotient (fdiv.h: Markstein's correction per quotient), which gives the
-// IEEE quotient bit for bit at about a third of the FP64 instructions of a division
-// per extra quotient; FP32: plain division, as the split path's flags compile it;
-// double-float: one double-word reciprocal and a double-word product per quotient
-// (relative error a few units of 2^-46, a third of a double-word division's cost).
+// Quotients by one divisor.  FP64: one reciprocal of the divisor serves every quotient,
+// all on the integer pipe (fdiv.h), each the IEEE quotient bit for bit; FP32: plain
+// division, as the split path's flags compile it; double-float: one double-word
+// reciprocal and a double-word product per quotient (relative error a few units of
+// 2^-46, a third of a double-word division's cost).
 template <typename T> struct Div {
     T b;
     __device__ __forceinline__ explicit Div(T d) : b(d) {}

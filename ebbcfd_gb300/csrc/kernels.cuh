@@ -35,6 +35,7 @@
 
 #include "bitconv.h"
 #include "device_math.cuh"
+#include "flux_soft.cuh"
 #include "layout.h"
 
 namespace ebbdev {
@@ -479,38 +480,18 @@ __device__ __forceinline__ void lp_limit(const DMesh &M, int i, int ne, const T 
     }
 }
 
-template <typename T, int MJ, bool LP, bool UNI, int PR>
-__global__ void __launch_bounds__(cell_threads<T, PR>(), cell_minb<T, PR>()) k_cell(DMesh M, DPhys P, DArrays A, const T *__restrict__ qin, int limit)
+// read-only mesh data of a cell loaded before the wait for the previous kernel (split
+// path): neighbour indices, gradient weights, neighbour and face midpoint offsets
+template <typename T, int MJ> struct CellPre {
+    int nb[MJ];
+    typename V2<T>::t gm[MJ], nd[MJ], fd[MJ];
+};
+
+template <typename T, int MJ, bool LP>
+__device__ __forceinline__ void cell_body(const DMesh &M, const DPhys &P, const DArrays &A, DState *st, int i, int ne,
+                                          const T *__restrict__ qin, int limit, CellPre<T, MJ> &pre)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool act = i < M.C;
     const int Cs = M.Cs;
-    // read-only mesh data first, before the wait for the previous kernel.  Split path:
-    // the neighbour rows are loaded whatever the cell's edge count (rows past it hold
-    // 0), and the limiter's and the reconstruction's geometry (neighbour and face
-    // midpoint offsets) is loaded here, not behind the gathers
-    int ne = 0, inst = 0;
-    int nbv[MJ];
-    typename V2<T>::t gmv[MJ], ndv[MJ], fdv[MJ];
-    if (act) {
-        ne = UNI ? MJ : M.nedge[i];  // UNI: every cell has MJ edges (all triangles, all quads)
-        if (M.cell_inst) inst = M.cell_inst[i];
-        if constexpr (sizeof(T) == 4) {
-#pragma unroll
-            for (int j = 0; j < MJ; j++) nbv[j] = M.s_nbr[(size_t)j * Cs + i];
-#pragma unroll
-            for (int j = 0; j < MJ; j++) {
-                gmv[j] = ld2<T>(M.g.s_gm, (size_t)j * Cs + i);
-                ndv[j] = ld2<T>(M.g.s_nd, (size_t)j * Cs + i);
-                fdv[j] = ld2<T>(M.g.s_fd, (size_t)j * Cs + i);
-            }
-        }
-    }
-    grid_dep_release();
-    grid_dep_wait();
-    if (!act) return;
-    DState *st = A.st + inst;
-    if (halted(st)) return;
     T *qghost = const_cast<T *>(qin);  // ghost slots [C, C+G) are written by their owner only
     T qi[4];
     ld4(qin + 4 * (size_t)i, qi);
@@ -527,15 +508,15 @@ __global__ void __launch_bounds__(cell_threads<T, PR>(), cell_minb<T, PR>()) k_c
         // all neighbour-state gathers in flight before any dependent math
         T qv[MJ][4];
 #pragma unroll
-        for (int j = 0; j < MJ; j++) nbv[j] = (j < ne) ? nbv[j] : i;
+        for (int j = 0; j < MJ; j++) pre.nb[j] = (j < ne) ? pre.nb[j] : i;
 #pragma unroll
-        for (int j = 0; j < MJ; j++) ld4(qin + 4 * (size_t)(nbv[j] < M.C ? nbv[j] : i), qv[j]);
+        for (int j = 0; j < MJ; j++) ld4(qin + 4 * (size_t)(pre.nb[j] < M.C ? pre.nb[j] : i), qv[j]);
 #pragma unroll
         for (int j = 0; j < MJ; j++) {
             if (j < ne) {
-                if (nbv[j] >= M.C) {
-                    ghost_state<T>(M, P, st, nbv[j] - M.C, qi, qv[j]);
-                    st4(qghost + 4 * (size_t)nbv[j], qv[j]);
+                if (pre.nb[j] >= M.C) {
+                    ghost_state<T>(M, P, st, pre.nb[j] - M.C, qi, qv[j]);
+                    st4(qghost + 4 * (size_t)pre.nb[j], qv[j]);
                 }
                 if (second) {
 #pragma unroll
@@ -543,8 +524,8 @@ __global__ void __launch_bounds__(cell_threads<T, PR>(), cell_minb<T, PR>()) k_c
                         mn[k] = fmin(mn[k], qv[j][k]);
                         mx[k] = fmax(mx[k], qv[j][k]);
                         T du = qv[j][k] - qi[k];
-                        g[k][0] = g[k][0] + gmv[j].x * du;
-                        g[k][1] = g[k][1] + gmv[j].y * du;
+                        g[k][0] = g[k][0] + pre.gm[j].x * du;
+                        g[k][1] = g[k][1] + pre.gm[j].y * du;
                     }
                 }
             }
@@ -699,7 +680,7 @@ __global__ void __launch_bounds__(cell_threads<T, PR>(), cell_minb<T, PR>()) k_c
             if (j < ne) {
                 typename V2<T>::t nd;
                 if constexpr (sizeof(T) == 4)
-                    nd = ndv[j];
+                    nd = pre.nd[j];
                 else
                     nd = ld2<T>(M.g.s_nd, (size_t)j * Cs + i);
                 // every pair's quotient is formed and selected (no divergent branch; the
@@ -757,7 +738,7 @@ __global__ void __launch_bounds__(cell_threads<T, PR>(), cell_minb<T, PR>()) k_c
             } else {
                 typename V2<T>::t fd;
                 if constexpr (sizeof(T) == 4)
-                    fd = fdv[j];
+                    fd = pre.fd[j];
                 else
                     fd = ld2<T>(M.g.s_fd, s);
 #pragma unroll
@@ -771,6 +752,275 @@ __global__ void __launch_bounds__(cell_threads<T, PR>(), cell_minb<T, PR>()) k_c
             }
             st4(face + 4 * s, f);
         }
+    }
+}
+
+// plain FP64: the cells cell_soft leaves
+template <typename T, int MJ, bool LP>
+__device__ __noinline__ void cell_plain(const DMesh &M, const DPhys &P, const DArrays &A, DState *st, int i, int ne,
+                                        const T *qin, int limit)
+{
+    CellPre<T, MJ> pre;
+    cell_body<T, MJ, LP>(M, P, A, st, i, ne, qin, limit, pre);
+}
+
+// The scalar limiter of one component (solve.d:336-402) on the integer and FP32 pipes.
+// dl <= 0 <= dh are the bounds minus the cell's value.  Which neighbours' extrapolations
+// leave the bounds, and which of those gives the smallest ratio, is decided in FP32 from
+// values truncated to 23 bits; a decision that is not clear of the truncation and rounding
+// errors sets `unsure` (limit_exact then decides; measured on smooth flows: 2 to 3 of
+// 1,000 cells).  Returns the deciding neighbour, or -1; `low` tells its bound.
+//
+// With dd = RN(RN(g0 nx) + RN(g1 ny)) and e its FP32 value: |e - dd| < 2^-21 (|a| + |b|),
+// the FP32 bounds are within 2^-23 of theirs, and RN(q + dd) compares with a bound as dd
+// does with its difference when they are 2^-51 |q| apart.
+template <int MJ>
+__device__ __forceinline__ int limiting_neighbour(double q, double g0, double g1, double dl, double dh,
+                                                  const float (&nx)[MJ], const float (&ny)[MJ], int ne, bool &low,
+                                                  bool &unsure)
+{
+    const float g0f = trunc_sat(g0), g1f = trunc_sat(g1), lo = trunc_sat(dl), hi = trunc_sat(dh);
+    const float M = __fadd_rn(0x1p-50f * fabsf(trunc_sat(q)), 0x1p-100f);
+    const float ml = __fmaf_rn(0x1p-21f, fabsf(lo), M), mh = __fmaf_rn(0x1p-21f, hi, M);
+    const float lo_out = lo - ml, lo_in = lo + ml, hi_out = hi + mh, hi_in = hi - mh;
+    const bool flat = g0 == 0.0 && g1 == 0.0;  // every extrapolation is the cell's value
+    int best = -1;
+    float s1 = 4.0f, up1 = 4.0f, dn1 = 4.0f, dn2 = 8.0f;  // the smallest ratio and its interval, the others' lower end
+#pragma unroll
+    for (int j = 0; j < MJ; j++) {
+        if (j < ne) {
+            const float a = __fmul_rn(g0f, nx[j]), b = __fmul_rn(g1f, ny[j]), e = __fadd_rn(a, b);
+            const float E = __fmul_rn(0x1p-20f, __fadd_rn(fabsf(a), fabsf(b)));
+            const float up = e + E, dn = e - E;
+            const bool below = up < lo_out, above = dn > hi_out, in = dn > lo_in && up < hi_in;
+            unsure |= !((below || above || in) && fabsf(e) < 0x1p100f) && !flat;
+            if (below || above) {
+                const float r = __fdividef(1.0f, e), s = (below ? lo : hi) * r;
+                const float w = s * __fmaf_rn(2.0f * E, fabsf(r), 0x1p-20f);
+                if (s < s1) {
+                    dn2 = fminf(dn2, dn1);
+                    s1 = s;
+                    up1 = s + w;
+                    dn1 = s - w;
+                    best = j;
+                    low = below;
+                } else {
+                    dn2 = fminf(dn2, s - w);
+                }
+            }
+        }
+    }
+    // two ratios too close to tell apart (a zero one is the smallest: its bound is exact)
+    if (best >= 0) unsure |= (low ? dl : dh) != 0.0 && !(s1 > 0x1p-60f && dn2 > up1);
+    return best;
+}
+
+// The limiter of component k in the reference's own expressions (solve.d:336-402), the
+// neighbours' values read again (ghosts as this thread has just written them).
+__device__ __forceinline__ double limit_exact(const DMesh &M, int i, int ne, const double *qin, int k, double q, double g0,
+                                              double g1)
+{
+    double mn = q, mx = q, l = 1.0;
+#pragma unroll 1
+    for (int j = 0; j < ne; j++) {
+        const double v = *(const volatile double *)(qin + 4 * (size_t)M.s_nbr[(size_t)j * M.Cs + i] + k);
+        mn = fmin(mn, v);
+        mx = fmax(mx, v);
+    }
+#pragma unroll 1
+    for (int j = 0; j < ne; j++) {
+        const double2 nd = ld2<double>(M.g.s_nd, (size_t)j * M.Cs + i);
+        const double dd = g0 * nd.x + g1 * nd.y, qE = q + dd;
+        if (qE < mn || qE > mx) l = fmin(l, ebbdiv::div((qE < mn ? mn : mx) - q, ebbdiv::recip(dd)));
+    }
+    return l;
+}
+
+// Gradient, scalar limiter and face states of a cell in FP64 with the products, the
+// limiter and its quotients on the integer and FP32 pipes (softdbl.h); the values are
+// cell_body's bit for bit.  False (and only ghost states written) where a value is out of
+// that arithmetic's range: the caller then runs cell_plain.
+//
+// What bounds it: the FP64 pipe still (61% busy), with the additions left and the limiter's
+// few products, which gain nothing on the integer pipe (143 against 148 us).  200,000
+// triangles: 52 us, 155 us with cell_plain's arithmetic; 400,000 plate cells: 143 and 318 us.
+template <int MJ>
+__device__ __forceinline__ bool cell_soft(const DMesh &M, const DPhys &P, const DArrays &A, DState *st, int i, int ne,
+                                          const double *__restrict__ qin, int limit)
+{
+    const int Cs = M.Cs;
+    bool bad = false;
+    double *qghost = const_cast<double *>(qin);  // ghost slots [C, C+G) are written by their owner only
+    double qi[4], g[4][2];
+    long long dlo[4], dhi[4];  // bit patterns of the smallest and largest neighbour difference
+    // the neighbour-state gathers in flight before the arithmetic
+    int nb[MJ];
+    double qv[MJ][4];
+#pragma unroll
+    for (int j = 0; j < MJ; j++) nb[j] = j < ne ? M.s_nbr[(size_t)j * Cs + i] : i;
+    ld4(qin + 4 * (size_t)i, qi);
+#pragma unroll
+    for (int j = 0; j < MJ; j++) ld4(qin + 4 * (size_t)(nb[j] < M.C ? nb[j] : i), qv[j]);
+#pragma unroll
+    for (int k = 0; k < 4; k++) dlo[k] = dhi[k] = 0;
+#pragma unroll
+    for (int j = 0; j < MJ; j++) {
+        if (j < ne) {
+            const size_t s = (size_t)j * Cs + i;
+            double *qn = qv[j];
+            if (nb[j] >= M.C) {
+                ghost_state<double>(M, P, st, nb[j] - M.C, qi, qn);
+                st4(qghost + 4 * (size_t)nb[j], qn);
+            }
+            const double2 gm = ld2<double>(M.g.s_gm, s);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const double du = qn[k] - qi[k];
+                ebbsoft::check<200>(du, bad);
+                // negative doubles are larger than others as unsigned integers, the more
+                // the larger their magnitude; non-negative ones order as signed integers
+                const long long bits = __double_as_longlong(du);
+                dlo[k] = (unsigned long long)bits > (unsigned long long)dlo[k] ? bits : dlo[k];
+                dhi[k] = bits > dhi[k] ? bits : dhi[k];
+                const double px = sm<SG_GRAD>(gm.x, du), py = sm<SG_GRAD>(gm.y, du);
+                g[k][0] = j == 0 ? zero_plus(px) : g[k][0] + px;
+                g[k][1] = j == 0 ? zero_plus(py) : g[k][1] + py;
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        ebbsoft::check<200>(g[k][0], bad);
+        ebbsoft::check<200>(g[k][1], bad);
+    }
+    double lim[4] = {1.0, 1.0, 1.0, 1.0}, lg[4][2];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        lg[k][0] = g[k][0];
+        lg[k][1] = g[k][1];
+    }
+    if (P.limited && limit) {
+        float nx[MJ], ny[MJ];
+#pragma unroll
+        for (int j = 0; j < MJ; j++) {
+            if (j < ne) {
+                const double2 nd = ld2<double>(M.g.s_nd, (size_t)j * Cs + i);
+                nx[j] = trunc_sat(nd.x);
+                ny[j] = trunc_sat(nd.y);
+            }
+        }
+        unsigned redo = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const double dl = dlo[k] < 0 ? __longlong_as_double(dlo[k]) : 0.0, dh = __longlong_as_double(dhi[k]);
+            bool low = false, unsure = false;
+            const int j = limiting_neighbour<MJ>(qi[k], g[k][0], g[k][1], dl, dh, nx, ny, ne, low, unsure);
+            if (unsure) {
+                redo |= 1u << k;
+            } else if (j >= 0) {
+                const double2 nd = ld2<double>(M.g.s_nd, (size_t)j * Cs + i);
+                const double dd = sm<SG_LIM>(g[k][0], nd.x) + sm<SG_LIM>(g[k][1], nd.y);
+                const double s = soft_ratio(low ? dl : dh, dd, bad);
+                lim[k] = __double2hiint(s) < 0x3ff00000 ? s : 1.0;  // min(1, s), s >= -0
+            }
+        }
+#pragma unroll 1
+        while (redo) {
+            const int k = __ffs(redo) - 1;
+            redo &= redo - 1;
+            double q = qi[0], g0 = g[0][0], g1 = g[0][1];
+#pragma unroll
+            for (int m = 1; m < 4; m++)
+                if (k == m) {
+                    q = qi[m];
+                    g0 = g[m][0];
+                    g1 = g[m][1];
+                }
+            const double l = limit_exact(M, i, ne, qin, k, q, g0, g1);
+#pragma unroll
+            for (int m = 0; m < 4; m++)
+                if (k == m) lim[m] = l;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            lg[k][0] = sm<SG_LIM>(lim[k], g[k][0]);
+            lg[k][1] = sm<SG_LIM>(lim[k], g[k][1]);
+            ebbsoft::check<400>(lg[k][0], bad);
+            ebbsoft::check<400>(lg[k][1], bad);
+        }
+    }
+    if (bad) return false;
+    if (P.need_grad) {
+        double *gp = reinterpret_cast<double *>(A.grad) + 8 * (size_t)i;
+        const double a[4] = {g[0][0], g[0][1], g[1][0], g[1][1]}, b[4] = {g[2][0], g[2][1], g[3][0], g[3][1]};
+        st4(gp, a);
+        st4(gp + 4, b);
+    }
+    if (A.lim) {
+        double *lp = reinterpret_cast<double *>(A.lim) + 8 * (size_t)i;
+        const double a[4] = {lim[0], lim[0], lim[1], lim[1]}, b[4] = {lim[2], lim[2], lim[3], lim[3]};
+        st4(lp, a);
+        st4(lp + 4, b);
+    }
+    double *face = reinterpret_cast<double *>(A.face);
+#pragma unroll
+    for (int j = 0; j < MJ; j++) {
+        if (j < ne) {
+            const size_t s = (size_t)j * Cs + i;
+            const double2 fd = ld2<double>(M.g.s_fd, s);
+            double f[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                f[k] = qi[k] + sm<SG_FACE>(lg[k][0], fd.x) + sm<SG_FACE>(lg[k][1], fd.y);
+            if (pressure_negative(f)) {
+                const double l = fmin(fmin(lim[0], lim[1]), fmin(lim[2], lim[3]));
+#pragma unroll
+                for (int k = 0; k < 4; k++) f[k] = qi[k] + l * g[k][0] * fd.x + l * g[k][1] * fd.y;
+            }
+            st4(face + 4 * s, f);
+        }
+    }
+    return true;
+}
+
+template <typename T, int MJ, bool LP, bool UNI, int PR>
+__global__ void __launch_bounds__(cell_threads<T, PR>(), cell_minb<T, PR>())
+    k_cell(const __grid_constant__ DMesh M, const __grid_constant__ DPhys P, const __grid_constant__ DArrays A,
+           const T *__restrict__ qin, int limit)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool act = i < M.C;
+    // read-only mesh data first, before the wait for the previous kernel.  Split path:
+    // the neighbour rows are loaded whatever the cell's edge count (rows past it hold
+    // 0), and the limiter's and the reconstruction's geometry (neighbour and face
+    // midpoint offsets) is loaded here, not behind the gathers
+    int ne = 0, inst = 0;
+    CellPre<T, MJ> pre;
+    if (act) {
+        ne = UNI ? MJ : M.nedge[i];  // UNI: every cell has MJ edges (all triangles, all quads)
+        if (M.cell_inst) inst = M.cell_inst[i];
+        if constexpr (sizeof(T) == 4) {
+            const int Cs = M.Cs;
+#pragma unroll
+            for (int j = 0; j < MJ; j++) pre.nb[j] = M.s_nbr[(size_t)j * Cs + i];
+#pragma unroll
+            for (int j = 0; j < MJ; j++) {
+                pre.gm[j] = ld2<T>(M.g.s_gm, (size_t)j * Cs + i);
+                pre.nd[j] = ld2<T>(M.g.s_nd, (size_t)j * Cs + i);
+                pre.fd[j] = ld2<T>(M.g.s_fd, (size_t)j * Cs + i);
+            }
+        }
+    }
+    grid_dep_release();
+    grid_dep_wait();
+    if (!act) return;
+    DState *st = A.st + inst;
+    if (halted(st)) return;
+    if constexpr (is_fp64<T> && !LP) {
+        if (!(M.soft && P.order > 1 && cell_soft<MJ>(M, P, A, st, i, UNI ? MJ : ne, qin, limit)))
+            cell_plain<T, MJ, LP>(M, P, A, st, i, ne, qin, limit);
+    } else {
+        cell_body<T, MJ, LP>(M, P, A, st, i, UNI ? MJ : ne, qin, limit, pre);
     }
 }
 
@@ -938,8 +1188,83 @@ __device__ void boundary_flux(const DMesh &M, const DPhys &P, const DArrays &A, 
     reinterpret_cast<T *>(A.fs)[e] = len * sMax;
 }
 
+// len * flux and len * sMax of interior edge e from its two face states (and, viscous,
+// its cells' gradients)
+template <typename T>
+__device__ __forceinline__ void edge_flux(const DMesh &M, const DPhys &P, const DArrays &A, DState *st, int inst, int e,
+                                          int2 sl, typename V2<T>::t n, T len)
+{
+    const T *face = reinterpret_cast<const T *>(A.face);
+    T qL[4], qR[4], F[4], sMax;
+    ld4(face + 4 * (size_t)sl.x, qL);
+    ld4(face + 4 * (size_t)sl.y, qR);
+    inviscid_flux(P.flux, qL, qR, n.x, n.y, F, sMax);
+    if (P.viscous) {
+        const int2 c = reinterpret_cast<const int2 *>(M.e_cell)[e];
+        T g1[4][2], g2[4][2], dq[4][2], qa[4], Fv[4];
+        load_grad<T>(A.grad, c.x, g1);
+        load_grad<T>(A.grad, c.y, g2);
+        for (int k = 0; k < 4; k++) {
+            qa[k] = half(qL[k] + qR[k]);
+            dq[k][0] = half(g1[k][0] + g2[k][0]);
+            dq[k][1] = half(g1[k][1] + g2[k][1]);
+        }
+        diffusive_flux(visc_const<T>(P), visc_mu<T>(M, P, inst), qa, dq, n.x, n.y, Fv);
+        for (int k = 0; k < 4; k++) F[k] = F[k] - Fv[k];
+    }
+    if (has_nan(F)) flag_error(st, 2, ERR_NAN_EDGE, (unsigned)M.e_ref[e]);
+    T lf[4] = {len * F[0], len * F[1], len * F[2], len * F[3]};
+    st4(reinterpret_cast<T *>(A.fl) + 4 * (size_t)e, lf);
+    reinterpret_cast<T *>(A.fs)[e] = len * sMax;
+}
+
+// plain FP64: the edges edge_flux_soft leaves
+template <typename T>
+__device__ __noinline__ void edge_flux_plain(const DMesh &M, const DPhys &P, const DArrays &A, DState *st, int inst, int e)
+{
+    edge_flux<T>(M, P, A, st, inst, e, reinterpret_cast<const int2 *>(M.e_slot)[e], ld2<T>(M.g.e_n, e),
+                 ld1<T>(M.g.e_len, e));
+}
+
+// edge_flux in FP64 with flux_soft.cuh's arithmetic; false (and nothing written) where
+// that does not hold for the edge's values.  No value here is a NaN.
+__device__ __forceinline__ bool edge_flux_soft(const DMesh &M, const DPhys &P, const DArrays &A, int inst, int e, int2 sl,
+                                               double2 n, double len)
+{
+    const double *face = reinterpret_cast<const double *>(A.face);
+    double qL[4], qR[4], F[4], sMax;  // F: twice the flux
+    bool bad = false;
+    ld4(face + 4 * (size_t)sl.x, qL);
+    ld4(face + 4 * (size_t)sl.y, qR);
+    inviscid_flux2_soft(P.flux, qL, qR, n.x, n.y, F, sMax, bad);
+    if (P.viscous) {
+        const int2 c = reinterpret_cast<const int2 *>(M.e_cell)[e];
+        double g1[4][2], g2[4][2], Fv[4];
+        load_grad<double>(A.grad, c.x, g1);
+        load_grad<double>(A.grad, c.y, g2);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            qL[k] = qL[k] + qR[k];
+            g1[k][0] = g1[k][0] + g2[k][0];
+            g1[k][1] = g1[k][1] + g2[k][1];
+        }
+        diffusive_flux2_soft(visc_const<double>(P), visc_mu<double>(M, P, inst), qL, g1, n.x, n.y, Fv, bad);
+        F[0] = F[0] - zero_dot(n.x, n.y);
+#pragma unroll
+        for (int k = 1; k < 4; k++) F[k] = F[k] - Fv[k];
+    }
+    if (bad) return false;
+    const double hl = 0.5 * len;
+    const double lf[4] = {hl * F[0], hl * F[1], hl * F[2], hl * F[3]};
+    st4(reinterpret_cast<double *>(A.fl) + 4 * (size_t)e, lf);
+    reinterpret_cast<double *>(A.fs)[e] = len * sMax;
+    return true;
+}
+
 template <typename T, int PR>
-__global__ void __launch_bounds__(flux_threads<T, PR>(), flux_minb<T, PR>()) k_flux(DMesh M, DPhys P, DArrays A, const T *__restrict__ qin, int nbi)
+__global__ void __launch_bounds__(flux_threads<T, PR>(), flux_minb<T, PR>())
+    k_flux(const __grid_constant__ DMesh M, const __grid_constant__ DPhys P, const __grid_constant__ DArrays A,
+           const T *__restrict__ qin, int nbi)
 {
     if ((int)blockIdx.x >= nbi) {
         grid_dep_release();
@@ -966,28 +1291,11 @@ __global__ void __launch_bounds__(flux_threads<T, PR>(), flux_minb<T, PR>()) k_f
     if (!act) return;
     DState *st = A.st + inst;
     if (halted(st)) return;
-    const T *face = reinterpret_cast<const T *>(A.face);
-    T qL[4], qR[4], F[4], sMax;
-    ld4(face + 4 * (size_t)sl.x, qL);
-    ld4(face + 4 * (size_t)sl.y, qR);
-    inviscid_flux(P.flux, qL, qR, n.x, n.y, F, sMax);
-    if (P.viscous) {
-        const int2 c = reinterpret_cast<const int2 *>(M.e_cell)[e];
-        T g1[4][2], g2[4][2], dq[4][2], qa[4], Fv[4];
-        load_grad<T>(A.grad, c.x, g1);
-        load_grad<T>(A.grad, c.y, g2);
-        for (int k = 0; k < 4; k++) {
-            qa[k] = half(qL[k] + qR[k]);
-            dq[k][0] = half(g1[k][0] + g2[k][0]);
-            dq[k][1] = half(g1[k][1] + g2[k][1]);
-        }
-        diffusive_flux(visc_const<T>(P), visc_mu<T>(M, P, inst), qa, dq, n.x, n.y, Fv);
-        for (int k = 0; k < 4; k++) F[k] = F[k] - Fv[k];
+    if constexpr (is_fp64<T>) {
+        if (!(M.soft && edge_flux_soft(M, P, A, inst, e, sl, n, len))) edge_flux_plain<T>(M, P, A, st, inst, e);
+    } else {
+        edge_flux<T>(M, P, A, st, inst, e, sl, n, len);
     }
-    if (has_nan(F)) flag_error(st, 2, ERR_NAN_EDGE, (unsigned)M.e_ref[e]);
-    T lf[4] = {len * F[0], len * F[1], len * F[2], len * F[3]};
-    st4(reinterpret_cast<T *>(A.fl) + 4 * (size_t)e, lf);
-    reinterpret_cast<T *>(A.fs)[e] = len * sMax;
 }
 
 // ---- fixed-order block reductions -------------------------------------------
@@ -1026,6 +1334,45 @@ __device__ __forceinline__ float warp_maxf(float v)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_down_sync(0xffffffffu, v, o));
     return v;
+}
+
+// o = a b for four values.  FP64: on the integer pipe where the values allow it (the
+// plain update kernel is bound by the FP64 pipe like the others: 76% busy, with 10% of
+// the issue slots used).
+template <typename T> __device__ __forceinline__ void mul4(const T a[4], T b, T o[4])
+{
+#pragma unroll
+    for (int k = 0; k < 4; k++) o[k] = a[k] * b;
+}
+template <> __device__ __forceinline__ void mul4<double>(const double a[4], double b, double o[4])
+{
+    bool bad = false;
+    ebbsoft::check<400>(b, bad);
+#pragma unroll
+    for (int k = 0; k < 4; k++) ebbsoft::check<400>(a[k], bad);
+    if (bad) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) o[k] = a[k] * b;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++) o[k] = ebbsoft::mul(a[k], b);
+    }
+}
+// a / b, FP64 on the integer pipe
+template <typename T> __device__ __forceinline__ T ratio(T a, T b) { return a / b; }
+template <> __device__ __forceinline__ double ratio<double>(double a, double b)
+{
+    return ebbdiv::div(a, ebbdiv::recip(b));
+}
+// acc + 2 x (2 x is exact: one rounding)
+template <typename T> __device__ __forceinline__ T plus_twice(T acc, T x) { return acc + T(2.0) * x; }
+template <> __device__ __forceinline__ double plus_twice<double>(double acc, double x) { return fma(2.0, x, acc); }
+// the larger of m and |x| for m >= 0; a NaN x leaves m
+__device__ __forceinline__ double max_abs(double m, double x)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+    const unsigned long long c = (unsigned long long)__double_as_longlong(m);
+    return b > c && b <= 0x7ff0000000000000ull ? __longlong_as_double((long long)b) : m;
 }
 
 // Residual of one interior cell and the stage combination.  The solution's update runs
@@ -1094,6 +1441,12 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
 #pragma unroll
         for (int j = 0; j < MJ; j++) {
             if (j < ne) {
+                if (is_fp64<T> && j == 0) {  // 0 + x without the FP64 pipe
+#pragma unroll
+                    for (int k = 0; k < 4; k++) r[k] = zero_plus(ev[0] < 0 ? -f[0][k] : f[0][k]);
+                    sAve = fe[0];
+                    continue;
+                }
                 if (ev[j] < 0) {
 #pragma unroll
                     for (int k = 0; k < 4; k++) r[k] = r[k] + (-f[j][k]);
@@ -1146,8 +1499,8 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
         }
         T *cdt = reinterpret_cast<T *>(A.cdt);
         if (need_dt || (P.local_ts && dt_update)) {
-            sAve /= ld1<T>(M.g.perim, i);
-            T c = (cfl_of<T>(st) * ld1<T>(M.g.dlen, i)) / sAve;
+            sAve = ratio(sAve, ld1<T>(M.g.perim, i));
+            T c = ratio(cfl_of<T>(st) * ld1<T>(M.g.dlen, i), sAve);
             if (need_dt) {
                 if (SPLIT)
                     fdtc = (float)c;
@@ -1168,13 +1521,11 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
             rm = to_f64(m);
         } else {
 #pragma unroll
-            for (int k = 0; k < 4; k++)
-                if ((double)fabs(r[k]) > rm) rm = (double)fabs(r[k]);
+            for (int k = 0; k < 4; k++) rm = max_abs(rm, r[k]);
         }
         const T s = ld1<T>(M.g.neg_inv_area, i);
         T R[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) R[k] = r[k] * s;
+        mul4(r, s, R);
         if (P.mms) {
             T S[4];
             ld4(ptr<T>(M.g.src) + 4 * (size_t)i, S);
@@ -1290,71 +1641,49 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
             for (int k = 0; k < 4; k++) Rd[k] = to_f64(R[k]);
             const double dt = st->dt;
             const double h = P.local_ts ? to_f64(cdt[i]) : dt;
-            if (ST == ST_EULER) {
+            double x[4], f = h, inc[4];  // the stage's increment is f x
 #pragma unroll
-                for (int k = 0; k < 4; k++) out[k] = q0[k] + h * Rd[k];
-            } else if (ST == ST_RK2_1) {
+            for (int k = 0; k < 4; k++) x[k] = Rd[k];
+            if (ST == ST_RK2_1) {
                 st4(aux + 4 * (size_t)i, R);
-#pragma unroll
-                for (int k = 0; k < 4; k++) out[k] = q0[k] + (dt * Rd[k]);
+                f = dt;
             } else if (ST == ST_RK2_2) {
                 T k1[4];
                 ld4(aux + 4 * (size_t)i, k1);
-                const double hh = P.local_ts ? h / 2.0 : st->dt_half;
-                if (SPLIT) {
 #pragma unroll
-                    for (int k = 0; k < 4; k++) out[k] = q0[k] + hh * ((double)k1[k] + Rd[k]);
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 4; k++) out[k] = q0[k] + hh * to_f64(k1[k] + R[k]);
-                }
-            } else if (ST == ST_TVD_1) {
-                if (SPLIT) st4(aux + 4 * (size_t)i, R);
-#pragma unroll
-                for (int k = 0; k < 4; k++) out[k] = q0[k] + h * Rd[k];
-            } else if (ST == ST_TVD_2) {
-                double qfe[4];
-                if (SPLIT) {  // recompute qFE = q + h R1 in FP64 from the FP32 R1
-                    T r1[4];
-                    ld4(aux + 4 * (size_t)i, r1);
-#pragma unroll
-                    for (int k = 0; k < 4; k++) qfe[k] = q0[k] + h * (double)r1[k];
-                } else {
-                    T qf[4];
-                    ld4(qin + 4 * (size_t)i, qf);
-#pragma unroll
-                    for (int k = 0; k < 4; k++) qfe[k] = to_f64(qf[k]);
-                }
-#pragma unroll
-                for (int k = 0; k < 4; k++) out[k] = 0.5 * (q0[k] + qfe[k] + h * Rd[k]);
+                for (int k = 0; k < 4; k++) x[k] = to_f64(k1[k] + R[k]);
+                f = P.local_ts ? h / 2.0 : st->dt_half;
             } else if (ST == ST_RK4_1) {
                 st4(aux + 4 * (size_t)i, R);
-#pragma unroll
-                for (int k = 0; k < 4; k++) out[k] = q0[k] + (st->dt_half * Rd[k]);
+                f = st->dt_half;
             } else if (ST == ST_RK4_2 || ST == ST_RK4_3) {
                 T acc[4];
                 ld4(aux + 4 * (size_t)i, acc);
 #pragma unroll
-                for (int k = 0; k < 4; k++) acc[k] = acc[k] + T(2.0) * R[k];
+                for (int k = 0; k < 4; k++) acc[k] = plus_twice(acc[k], R[k]);
                 st4(aux + 4 * (size_t)i, acc);
-                if (ST == ST_RK4_2) {
-#pragma unroll
-                    for (int k = 0; k < 4; k++) out[k] = q0[k] + (st->dt_half * Rd[k]);
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 4; k++) out[k] = q0[k] + (dt * Rd[k]);
-                }
-            } else {  // ST_RK4_4
+                f = ST == ST_RK4_2 ? st->dt_half : dt;
+            } else if (ST == ST_RK4_4) {
                 T acc[4];
                 ld4(aux + 4 * (size_t)i, acc);
-                const double hh = P.local_ts ? h / 6.0 : st->dt_sixth;
-                if (SPLIT) {
 #pragma unroll
-                    for (int k = 0; k < 4; k++) out[k] = q0[k] + hh * ((double)acc[k] + Rd[k]);
-                } else {
+                for (int k = 0; k < 4; k++) x[k] = to_f64(acc[k] + R[k]);
+                f = P.local_ts ? ratio(h, 6.0) : st->dt_sixth;
+            }
+            if constexpr (is_fp64<T>) {
+                mul4(x, f, inc);
+            } else {
 #pragma unroll
-                    for (int k = 0; k < 4; k++) out[k] = q0[k] + hh * to_f64(acc[k] + R[k]);
-                }
+                for (int k = 0; k < 4; k++) inc[k] = f * x[k];  // contracted with the sum below
+            }
+            if (ST == ST_TVD_2) {
+                T qf[4];
+                ld4(qin + 4 * (size_t)i, qf);
+#pragma unroll
+                for (int k = 0; k < 4; k++) out[k] = half(q0[k] + to_f64(qf[k]) + inc[k]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; k++) out[k] = q0[k] + inc[k];
             }
             if (final_stage) {
                 st4(A.q64 + 4 * (size_t)i, out);
