@@ -34,7 +34,7 @@ namespace ebbdev {
 constexpr int SG_SIDE = 0, SG_CONV = 1, SG_MEAN = 2, SG_WAVE = 3, SG_VMAT = 4, SG_VSUM = 5, SG_OUT = 6, SG_GRAD = 7,
               SG_LIM = 8, SG_FACE = 9;
 #ifndef EBB_SOFT_GROUPS
-#define EBB_SOFT_GROUPS 0x2ff
+#define EBB_SOFT_GROUPS 0x3ff
 #endif
 template <int GROUP> __device__ __forceinline__ double sm(double a, double b)
 {

@@ -111,6 +111,21 @@ template <typename T, int PR> constexpr int upd_minb()
 {
     return pick<T, PR>(EBB_UPD_MINB_F, EBB_UPD_MINB_FI, EBB_UPD_MINB_D, EBB_UPD_MINB_W);
 }
+// k_cell4 (four threads per cell)
+#ifndef EBB_CELL4_TB_D
+#define EBB_CELL4_TB_D 128
+#endif
+#ifndef EBB_CELL4_MINB_D
+#define EBB_CELL4_MINB_D 8
+#endif
+#ifndef EBB_CELL4_TB_W
+#define EBB_CELL4_TB_W 128
+#endif
+#ifndef EBB_CELL4_MINB_W
+#define EBB_CELL4_MINB_W 8
+#endif
+template <typename T> constexpr int cell4_threads() { return is_fp64<T> ? EBB_CELL4_TB_D : EBB_CELL4_TB_W; }
+template <typename T> constexpr int cell4_minb() { return is_fp64<T> ? EBB_CELL4_MINB_D : EBB_CELL4_MINB_W; }
 // an SM holds at most 2048 threads: every (threads, minimum blocks) pair must fit
 static_assert(EBB_CELL_TB_F * EBB_CELL_MINB_F <= 2048 && EBB_CELL_TB_D * EBB_CELL_MINB_D <= 2048 &&
                   EBB_CELL_TB_FI * EBB_CELL_MINB_FI <= 2048,
@@ -755,7 +770,7 @@ __device__ __forceinline__ void cell_body(const DMesh &M, const DPhys &P, const 
     }
 }
 
-// plain FP64: the cells cell_soft leaves
+// plain FP64: the cells k_cell4 leaves
 template <typename T, int MJ, bool LP>
 __device__ __noinline__ void cell_plain(const DMesh &M, const DPhys &P, const DArrays &A, DState *st, int i, int ne,
                                         const T *qin, int limit)
@@ -836,151 +851,233 @@ __device__ __forceinline__ double limit_exact(const DMesh &M, int i, int ne, con
     return l;
 }
 
-// Gradient, scalar limiter and face states of a cell in FP64 with the products, the
-// limiter and its quotients on the integer and FP32 pipes (softdbl.h); the values are
-// cell_body's bit for bit.  False (and only ghost states written) where a value is out of
-// that arithmetic's range: the caller then runs cell_plain.
-//
-// What bounds it: the FP64 pipe still (61% busy), with the additions left and the limiter's
-// few products, which gain nothing on the integer pipe (143 against 148 us).  200,000
-// triangles: 52 us, 155 us with cell_plain's arithmetic; 400,000 plate cells: 143 and 318 us.
-template <int MJ>
-__device__ __forceinline__ bool cell_soft(const DMesh &M, const DPhys &P, const DArrays &A, DState *st, int i, int ne,
-                                          const double *__restrict__ qin, int limit)
+// pressure_negative of a face state whose four components sit in the four lanes of a
+// quad (x: this lane's, k its index), the same answer in each of them
+__device__ __forceinline__ bool pressure_negative4(double x, int k, unsigned quad)
 {
+    const bool ok = (k == 0 || k == 3) ? mid_range(x, true) : f32_range(x);
+    const float t = ok ? trunc_sat(x) : NAN;
+    const float r = __shfl_sync(quad, t, 0, 4), m1 = __shfl_sync(quad, t, 1, 4), m2 = __shfl_sync(quad, t, 2, 4),
+                e = __shfl_sync(quad, t, 3, 4);
+    const float W = __fmul_rn(e, r), Z = __fmul_rn(0.5f, __fadd_rn(__fmul_rn(m1, m1), __fmul_rn(m2, m2)));
+    const float d = __fsub_rn(W, Z);
+    if (fabsf(d) > 0x1p-17f * __fadd_rn(fabsf(W), Z)) return d < 0.0f;
+    const double q[4] = {__shfl_sync(quad, x, 0, 4), __shfl_sync(quad, x, 1, 4), __shfl_sync(quad, x, 2, 4),
+                         __shfl_sync(quad, x, 3, 4)};
+    return pressure_negative(q);
+}
+__device__ __forceinline__ df shfl4(unsigned quad, df x, int k)
+{
+    return df(__shfl_sync(quad, x.hi, k, 4), __shfl_sync(quad, x.lo, k, 4));
+}
+__device__ __forceinline__ double shfl4(unsigned quad, double x, int k) { return __shfl_sync(quad, x, k, 4); }
+__device__ __forceinline__ bool pressure_negative4(df x, int, unsigned quad)
+{
+    const float r = __shfl_sync(quad, x.hi, 0, 4), m1 = __shfl_sync(quad, x.hi, 1, 4), m2 = __shfl_sync(quad, x.hi, 2, 4),
+                e = __shfl_sync(quad, x.hi, 3, 4);
+    const float W = e * r, Z = 0.5f * (m1 * m1 + m2 * m2), d = W - Z;
+    if (r > 0.0f && fabsf(d) > 0x1p-17f * (fabsf(W) + Z) + 0x1p-100f) return d < 0.0f;
+    const df q[4] = {shfl4(quad, x, 0), shfl4(quad, x, 1), shfl4(quad, x, 2), shfl4(quad, x, 3)};
+    return pressure_negative(q);
+}
+
+// Gradient, scalar limiter and face states with four threads per cell, one per component
+// (plain FP64 and double-float; second order, without the LP limiter).  The components
+// meet only in the ghost states and the pressure test of a face, so a thread carries a
+// quarter of the values: the registers of one thread per cell (80 and 128 of them) kept
+// 24 and 16 warps on an SM, too few to cover the latency of either form's arithmetic.
+//
+// FP64: the products, the limiter's decisions and its quotients run on the integer and
+// FP32 pipes (softdbl.h) beside the FP64 pipe; the values are cell_body's bit for bit,
+// and a cell with a value out of that arithmetic's range goes to cell_plain.  Bound by
+// the FP64 pipe's additions (61% busy; integer pipe 50%, a sixth of the time fetching
+// instructions).  Double-float: issue (66% of the slots).
+//
+// Lane k loads the geometry of slot k before the wait for the previous kernel: with each
+// lane loading every slot's where it is used, loads from memory took 45% (FP64) and 63%
+// (double-float) of the warps' time.
+//
+// Measured against one thread per cell, us per launch, FP64 / double-float: 400,000 plate
+// cells 140 (143) / 84 (109); 200,000 triangles 53 (52) / 28 (36); 1024 quads, where one
+// warp's latency is the launch's, 7.5 (16.3) / 5.6 (14.1).  FP64 steps: 1,815 (1,879),
+// 318 (329) and 76 (91) us.
+template <typename T, int MJ, bool UNI>
+__global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
+    k_cell4(const __grid_constant__ DMesh M, const __grid_constant__ DPhys P, const __grid_constant__ DArrays A,
+            const T *__restrict__ qin, int limit)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = t >> 2, k = t & 3;
+    const bool act = i < M.C;
     const int Cs = M.Cs;
-    bool bad = false;
-    double *qghost = const_cast<double *>(qin);  // ghost slots [C, C+G) are written by their owner only
-    double qi[4], g[4][2];
-    long long dlo[4], dhi[4];  // bit patterns of the smallest and largest neighbour difference
-    // the neighbour-state gathers in flight before the arithmetic
+    // read-only mesh data before the wait for the previous kernel: lane k holds the slots
+    // k and k + 4 of its cell (rows past the cell's edges hold 0), so that every load is in
+    // flight at once; the quad passes them around
+    constexpr int H = MJ > 4 ? 2 : 1;
+    int ne = 0, inst = 0, nbk[H] = {};
+    typename V2<T>::t gmk[H] = {}, ndk[H] = {}, fdk[H] = {};
+    if (act) {
+        ne = UNI ? MJ : M.nedge[i];
+        if (M.cell_inst) inst = M.cell_inst[i];
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            if (4 * h + k < MJ) {
+                const size_t s = (size_t)(4 * h + k) * Cs + i;
+                nbk[h] = M.s_nbr[s];
+                gmk[h] = ld2<T>(M.g.s_gm, s);
+                ndk[h] = ld2<T>(M.g.s_nd, s);
+                fdk[h] = ld2<T>(M.g.s_fd, s);
+            }
+        }
+    }
+    grid_dep_release();
+    grid_dep_wait();
+    if (!act) return;  // a quad's lanes agree here and below
+    DState *st = A.st + inst;
+    if (halted(st)) return;
+    const unsigned quad = 0xfu << (threadIdx.x & 28);
+    T *qghost = const_cast<T *>(qin);  // ghost slots [C, C+G) are written by their owner only
+    const T qi = qin[4 * (size_t)i + k];
     int nb[MJ];
-    double qv[MJ][4];
-#pragma unroll
-    for (int j = 0; j < MJ; j++) nb[j] = j < ne ? M.s_nbr[(size_t)j * Cs + i] : i;
-    ld4(qin + 4 * (size_t)i, qi);
-#pragma unroll
-    for (int j = 0; j < MJ; j++) ld4(qin + 4 * (size_t)(nb[j] < M.C ? nb[j] : i), qv[j]);
-#pragma unroll
-    for (int k = 0; k < 4; k++) dlo[k] = dhi[k] = 0;
+    T qv[MJ];
 #pragma unroll
     for (int j = 0; j < MJ; j++) {
-        if (j < ne) {
-            const size_t s = (size_t)j * Cs + i;
-            double *qn = qv[j];
-            if (nb[j] >= M.C) {
-                ghost_state<double>(M, P, st, nb[j] - M.C, qi, qn);
-                st4(qghost + 4 * (size_t)nb[j], qn);
-            }
-            const double2 gm = ld2<double>(M.g.s_gm, s);
+        nb[j] = __shfl_sync(quad, nbk[j >> 2], j & 3, 4);
+        if (UNI || j < ne) qv[j] = qin[4 * (size_t)(nb[j] < M.C ? nb[j] : i) + k];
+    }
+    auto slot = [&](const typename V2<T>::t(&v)[H], int j) {  // slot j's pair, j a constant
+        typename V2<T>::t o;
+        o.x = shfl4(quad, v[j >> 2].x, j & 3);
+        o.y = shfl4(quad, v[j >> 2].y, j & 3);
+        return o;
+    };
+    bool bad = false;
+    T g0 = T(0.0), g1 = T(0.0), mn = qi, mx = qi;
+    long long dlo = 0, dhi = 0;  // FP64: bit patterns of the smallest and largest neighbour difference
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const double du = qn[k] - qi[k];
+    for (int j = 0; j < MJ; j++) {
+        if (UNI || j < ne) {
+            if (nb[j] >= M.C) {
+                const T q[4] = {shfl4(quad, qi, 0), shfl4(quad, qi, 1), shfl4(quad, qi, 2), shfl4(quad, qi, 3)};
+                T gh[4];
+                ghost_state<T>(M, P, st, nb[j] - M.C, q, gh);
+                qv[j] = k < 2 ? (k ? gh[1] : gh[0]) : (k == 2 ? gh[2] : gh[3]);
+                qghost[4 * (size_t)nb[j] + k] = qv[j];
+            }
+            const typename V2<T>::t gm = slot(gmk, j);
+            const T du = qv[j] - qi;
+            if constexpr (is_fp64<T>) {
                 ebbsoft::check<200>(du, bad);
                 // negative doubles are larger than others as unsigned integers, the more
                 // the larger their magnitude; non-negative ones order as signed integers
                 const long long bits = __double_as_longlong(du);
-                dlo[k] = (unsigned long long)bits > (unsigned long long)dlo[k] ? bits : dlo[k];
-                dhi[k] = bits > dhi[k] ? bits : dhi[k];
+                dlo = (unsigned long long)bits > (unsigned long long)dlo ? bits : dlo;
+                dhi = bits > dhi ? bits : dhi;
                 const double px = sm<SG_GRAD>(gm.x, du), py = sm<SG_GRAD>(gm.y, du);
-                g[k][0] = j == 0 ? zero_plus(px) : g[k][0] + px;
-                g[k][1] = j == 0 ? zero_plus(py) : g[k][1] + py;
+                g0 = j == 0 ? zero_plus(px) : g0 + px;
+                g1 = j == 0 ? zero_plus(py) : g1 + py;
+            } else {
+                mn = fmin(mn, qv[j]);
+                mx = fmax(mx, qv[j]);
+                g0 = g0 + gm.x * du;
+                g1 = g1 + gm.y * du;
             }
         }
     }
+    T lim = T(1.0);
+    if constexpr (is_fp64<T>) {
+        ebbsoft::check<200>(g0, bad);
+        ebbsoft::check<200>(g1, bad);
+        if (P.limited && limit) {
+            float nx[MJ], ny[MJ], nxk[H], nyk[H];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        ebbsoft::check<200>(g[k][0], bad);
-        ebbsoft::check<200>(g[k][1], bad);
-    }
-    double lim[4] = {1.0, 1.0, 1.0, 1.0}, lg[4][2];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        lg[k][0] = g[k][0];
-        lg[k][1] = g[k][1];
-    }
-    if (P.limited && limit) {
-        float nx[MJ], ny[MJ];
-#pragma unroll
-        for (int j = 0; j < MJ; j++) {
-            if (j < ne) {
-                const double2 nd = ld2<double>(M.g.s_nd, (size_t)j * Cs + i);
-                nx[j] = trunc_sat(nd.x);
-                ny[j] = trunc_sat(nd.y);
+            for (int h = 0; h < H; h++) {
+                nxk[h] = trunc_sat(ndk[h].x);
+                nyk[h] = trunc_sat(ndk[h].y);
             }
-        }
-        unsigned redo = 0;
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const double dl = dlo[k] < 0 ? __longlong_as_double(dlo[k]) : 0.0, dh = __longlong_as_double(dhi[k]);
+            for (int j = 0; j < MJ; j++) {
+                nx[j] = __shfl_sync(quad, nxk[j >> 2], j & 3, 4);
+                ny[j] = __shfl_sync(quad, nyk[j >> 2], j & 3, 4);
+            }
+            const double dl = dlo < 0 ? __longlong_as_double(dlo) : 0.0, dh = __longlong_as_double(dhi);
             bool low = false, unsure = false;
-            const int j = limiting_neighbour<MJ>(qi[k], g[k][0], g[k][1], dl, dh, nx, ny, ne, low, unsure);
+            const int j = limiting_neighbour<MJ>(qi, g0, g1, dl, dh, nx, ny, UNI ? MJ : ne, low, unsure);
             if (unsure) {
-                redo |= 1u << k;
+                lim = limit_exact(M, i, UNI ? MJ : ne, qin, k, qi, g0, g1);
             } else if (j >= 0) {
                 const double2 nd = ld2<double>(M.g.s_nd, (size_t)j * Cs + i);
-                const double dd = sm<SG_LIM>(g[k][0], nd.x) + sm<SG_LIM>(g[k][1], nd.y);
+                const double dd = sm<SG_LIM>(g0, nd.x) + sm<SG_LIM>(g1, nd.y);
                 const double s = soft_ratio(low ? dl : dh, dd, bad);
-                lim[k] = __double2hiint(s) < 0x3ff00000 ? s : 1.0;  // min(1, s), s >= -0
+                lim = __double2hiint(s) < 0x3ff00000 ? s : 1.0;  // min(1, s), s >= -0
             }
         }
-#pragma unroll 1
-        while (redo) {
-            const int k = __ffs(redo) - 1;
-            redo &= redo - 1;
-            double q = qi[0], g0 = g[0][0], g1 = g[0][1];
+    } else if (P.limited && limit) {
+        // which extrapolations leave the bounds first, then only their quotients
+        unsigned need = 0, above = 0;
 #pragma unroll
-            for (int m = 1; m < 4; m++)
-                if (k == m) {
-                    q = qi[m];
-                    g0 = g[m][0];
-                    g1 = g[m][1];
-                }
-            const double l = limit_exact(M, i, ne, qin, k, q, g0, g1);
-#pragma unroll
-            for (int m = 0; m < 4; m++)
-                if (k == m) lim[m] = l;
+        for (int j = 0; j < MJ; j++) {
+            if (UNI || j < ne) {
+                const typename V2<T>::t nd = slot(ndk, j);
+                const T qE = qi + (g0 * nd.x + g1 * nd.y);
+                const bool lo = qE < mn, hi = qE > mx;
+                if (lo || hi) need |= 1u << j;
+                if (!lo && hi) above |= 1u << j;
+            }
         }
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            lg[k][0] = sm<SG_LIM>(lim[k], g[k][0]);
-            lg[k][1] = sm<SG_LIM>(lim[k], g[k][1]);
-            ebbsoft::check<400>(lg[k][0], bad);
-            ebbsoft::check<400>(lg[k][1], bad);
+        while (need) {
+            const int j = __ffs(need) - 1;
+            need &= need - 1;
+            const typename V2<T>::t nd = ld2<T>(M.g.s_nd, (size_t)j * Cs + i);
+            lim = fmin(lim, ((above >> j & 1u) ? mx - qi : mn - qi) / (g0 * nd.x + g1 * nd.y));
         }
     }
-    if (bad) return false;
+    T lg0, lg1;
+    if constexpr (is_fp64<T>) {
+        lg0 = sm<SG_LIM>(lim, g0);
+        lg1 = sm<SG_LIM>(lim, g1);
+        ebbsoft::check<400>(lg0, bad);
+        ebbsoft::check<400>(lg1, bad);
+        if (__any_sync(quad, bad)) {
+            if (k == 0) cell_plain<T, MJ, false>(M, P, A, st, i, ne, qin, limit);
+            return;
+        }
+    } else {
+        lg0 = lim * g0;
+        lg1 = lim * g1;
+    }
+    typename V2<T>::t pair;
     if (P.need_grad) {
-        double *gp = reinterpret_cast<double *>(A.grad) + 8 * (size_t)i;
-        const double a[4] = {g[0][0], g[0][1], g[1][0], g[1][1]}, b[4] = {g[2][0], g[2][1], g[3][0], g[3][1]};
-        st4(gp, a);
-        st4(gp + 4, b);
+        pair.x = g0;
+        pair.y = g1;
+        reinterpret_cast<typename V2<T>::t *>(A.grad)[4 * (size_t)i + k] = pair;
     }
-    if (A.lim) {
-        double *lp = reinterpret_cast<double *>(A.lim) + 8 * (size_t)i;
-        const double a[4] = {lim[0], lim[0], lim[1], lim[1]}, b[4] = {lim[2], lim[2], lim[3], lim[3]};
-        st4(lp, a);
-        st4(lp + 4, b);
+    if (A.lim) {  // limiter values, exported for ebb-reconstruct
+        pair.x = lim;
+        pair.y = lim;
+        reinterpret_cast<typename V2<T>::t *>(A.lim)[4 * (size_t)i + k] = pair;
     }
-    double *face = reinterpret_cast<double *>(A.face);
+    T *face = reinterpret_cast<T *>(A.face);
 #pragma unroll
     for (int j = 0; j < MJ; j++) {
-        if (j < ne) {
+        if (UNI || j < ne) {
             const size_t s = (size_t)j * Cs + i;
-            const double2 fd = ld2<double>(M.g.s_fd, s);
-            double f[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-                f[k] = qi[k] + sm<SG_FACE>(lg[k][0], fd.x) + sm<SG_FACE>(lg[k][1], fd.y);
-            if (pressure_negative(f)) {
-                const double l = fmin(fmin(lim[0], lim[1]), fmin(lim[2], lim[3]));
-#pragma unroll
-                for (int k = 0; k < 4; k++) f[k] = qi[k] + l * g[k][0] * fd.x + l * g[k][1] * fd.y;
+            const typename V2<T>::t fd = slot(fdk, j);
+            T f;
+            if constexpr (is_fp64<T>)
+                f = qi + sm<SG_FACE>(lg0, fd.x) + sm<SG_FACE>(lg1, fd.y);
+            else
+                f = qi + lg0 * fd.x + lg1 * fd.y;
+            if (pressure_negative4(f, k, quad)) {
+                T l = fmin(T(1.0), shfl4(quad, lim, 0));
+                l = fmin(l, shfl4(quad, lim, 1));
+                l = fmin(l, shfl4(quad, lim, 2));
+                l = fmin(l, shfl4(quad, lim, 3));
+                f = qi + l * g0 * fd.x + l * g1 * fd.y;
             }
-            st4(face + 4 * s, f);
+            face[4 * s + k] = f;
         }
     }
-    return true;
 }
 
 template <typename T, int MJ, bool LP, bool UNI, int PR>
@@ -1016,12 +1113,7 @@ __global__ void __launch_bounds__(cell_threads<T, PR>(), cell_minb<T, PR>())
     if (!act) return;
     DState *st = A.st + inst;
     if (halted(st)) return;
-    if constexpr (is_fp64<T> && !LP) {
-        if (!(M.soft && P.order > 1 && cell_soft<MJ>(M, P, A, st, i, UNI ? MJ : ne, qin, limit)))
-            cell_plain<T, MJ, LP>(M, P, A, st, i, ne, qin, limit);
-    } else {
-        cell_body<T, MJ, LP>(M, P, A, st, i, UNI ? MJ : ne, qin, limit, pre);
-    }
+    cell_body<T, MJ, LP>(M, P, A, st, i, UNI ? MJ : ne, qin, limit, pre);
 }
 
 template <typename T> __device__ __forceinline__ void load_grad(const void *grad, int c, T g[4][2])
@@ -1820,6 +1912,22 @@ int launch_cell_pr(const DMesh &M, const DPhys &P, const DArrays &A, const T *qi
     cudaStream_t s = (cudaStream_t)stream;
     const bool lp = P.lp && P.limited;
     cudaError_t e;
+    if constexpr (!is_fp32<T>) {
+        // four threads per cell wherever k_cell4 holds: every mesh size is faster with it
+        if (!lp && P.order > 1 && (M.soft || !is_fp64<T>)) {
+            const int T4 = cell4_threads<T>();
+            const dim3 g4((unsigned)((4 * (int64_t)M.C + T4 - 1) / T4)), b4(T4);
+            if (M.maxJ <= 3)
+                e = M.uniform ? launch_dep(k_cell4<T, 3, true>, g4, b4, s, M, P, A, qin, limit)
+                              : launch_dep(k_cell4<T, 3, false>, g4, b4, s, M, P, A, qin, limit);
+            else if (M.maxJ == 4)
+                e = M.uniform ? launch_dep(k_cell4<T, 4, true>, g4, b4, s, M, P, A, qin, limit)
+                              : launch_dep(k_cell4<T, 4, false>, g4, b4, s, M, P, A, qin, limit);
+            else
+                e = launch_dep(k_cell4<T, 6, false>, g4, b4, s, M, P, A, qin, limit);
+            return ret(e);
+        }
+    }
 #define EBB_CELL_U(MJ, U)                                                                 \
     if (lp)                                                                               \
         e = launch_dep(k_cell<T, MJ, true, U, PR>, grid, dim3(TB), s, M, P, A, qin, limit); \
