@@ -2,8 +2,9 @@
 // gradient and limiter arithmetic on (hi, lo) pairs of FP32 numbers (dfloat.h, ~46
 // significant bits) on the FP32 pipe, which GB300 runs at 64 times its FP64 rate; the
 // solution update and the reductions inside k_update run in FP64 as on the plain path.
-// Compiled with IEEE FP32 division and square root and FP32 denormals kept: the
-// double-word algorithms need every FP32 operation correctly rounded.
+// Compiled with IEEE FP32 division and square root, FP32 denormals kept and no multiply-add
+// contraction: the double-word algorithms need every FP32 operation correctly rounded, as
+// written.
 #include "kernels.cuh"
 
 EBB_INSTANTIATE(ebbdf::df)

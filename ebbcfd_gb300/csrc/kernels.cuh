@@ -35,6 +35,7 @@
 
 #include "bitconv.h"
 #include "device_math.cuh"
+#include "flux_df.cuh"
 #include "flux_soft.cuh"
 #include "layout.h"
 
@@ -1310,6 +1311,42 @@ __device__ __forceinline__ void edge_flux(const DMesh &M, const DPhys &P, const 
     reinterpret_cast<T *>(A.fs)[e] = len * sMax;
 }
 
+// edge_flux in double-float with flux_df.cuh's packed arithmetic
+__device__ __forceinline__ void edge_flux_df(const DMesh &M, const DPhys &P, const DArrays &A, DState *st, int inst, int e,
+                                             int2 sl, df2 n, df len)
+{
+    const df *face = reinterpret_cast<const df *>(A.face);
+    df qL[4], qR[4], sMax;
+    dfp F03, F12;
+    ld4(face + 4 * (size_t)sl.x, qL);
+    ld4(face + 4 * (size_t)sl.y, qR);
+    if (P.flux == 1)
+        roe_flux_df(qL, qR, n.x, n.y, F03, F12, sMax);
+    else
+        rusanov_flux_df(qL, qR, n.x, n.y, F03, F12, sMax);
+    if (P.viscous) {
+        const int2 c = reinterpret_cast<const int2 *>(M.e_cell)[e];
+        df g1[4][2], g2[4][2], qa[4], o3;
+        dfp dq[4], o12;
+        load_grad<df>(A.grad, c.x, g1);
+        load_grad<df>(A.grad, c.y, g2);
+#pragma unroll
+        for (int k = 0; k < 4; k++) dq[k] = half(pair(g1[k][0], g1[k][1]) + pair(g2[k][0], g2[k][1]));
+        split(half(pair(qL[0], qL[1]) + pair(qR[0], qR[1])), qa[0], qa[1]);
+        split(half(pair(qL[2], qL[3]) + pair(qR[2], qR[3])), qa[2], qa[3]);
+        diffusive_flux_df(visc_const<df>(P), visc_mu<df>(M, P, inst), qa, dq, n.x, n.y, o3, o12);
+        F03 = F03 - pair(df(0.0f), o3);
+        F12 = F12 - o12;
+    }
+    const dfp l = both(len), a = l * F03, b = l * F12;
+    df f[4];
+    split(a, f[0], f[3]);
+    split(b, f[1], f[2]);
+    if (has_nan(f)) flag_error(st, 2, ERR_NAN_EDGE, (unsigned)M.e_ref[e]);
+    st4(reinterpret_cast<df *>(A.fl) + 4 * (size_t)e, f);
+    reinterpret_cast<df *>(A.fs)[e] = len * sMax;
+}
+
 // plain FP64: the edges edge_flux_soft leaves
 template <typename T>
 __device__ __noinline__ void edge_flux_plain(const DMesh &M, const DPhys &P, const DArrays &A, DState *st, int inst, int e)
@@ -1385,6 +1422,8 @@ __global__ void __launch_bounds__(flux_threads<T, PR>(), flux_minb<T, PR>())
     if (halted(st)) return;
     if constexpr (is_fp64<T>) {
         if (!(M.soft && edge_flux_soft(M, P, A, inst, e, sl, n, len))) edge_flux_plain<T>(M, P, A, st, inst, e);
+    } else if constexpr (is_df<T>) {
+        edge_flux_df(M, P, A, st, inst, e, sl, n, len);
     } else {
         edge_flux<T>(M, P, A, st, inst, e, sl, n, len);
     }
@@ -1762,20 +1801,15 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
                 for (int k = 0; k < 4; k++) x[k] = to_f64(acc[k] + R[k]);
                 f = P.local_ts ? ratio(h, 6.0) : st->dt_sixth;
             }
-            if constexpr (is_fp64<T>) {
-                mul4(x, f, inc);
-            } else {
+            if constexpr (is_fp64<T>) mul4(x, f, inc);
+            T qf[4];
+            if (ST == ST_TVD_2) ld4(qin + 4 * (size_t)i, qf);
 #pragma unroll
-                for (int k = 0; k < 4; k++) inc[k] = f * x[k];  // contracted with the sum below
-            }
-            if (ST == ST_TVD_2) {
-                T qf[4];
-                ld4(qin + 4 * (size_t)i, qf);
-#pragma unroll
-                for (int k = 0; k < 4; k++) out[k] = half(q0[k] + to_f64(qf[k]) + inc[k]);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 4; k++) out[k] = q0[k] + inc[k];
+            for (int k = 0; k < 4; k++) {
+                const double b = ST == ST_TVD_2 ? q0[k] + to_f64(qf[k]) : q0[k];
+                // the reference's two roundings on the plain path, one on the double-float path
+                out[k] = is_fp64<T> ? b + inc[k] : fma(f, x[k], b);
+                if (ST == ST_TVD_2) out[k] = half(out[k]);
             }
             if (final_stage) {
                 st4(A.q64 + 4 * (size_t)i, out);
