@@ -374,7 +374,7 @@ size_t bytes_of(const Dims &D, int32_t precision)
     total += 2 * rsz(4 * NQ);                              // qs, aux
     total += rsz(4 * MJ * Cs) + rsz(8 * NQ);               // face, grad
     total += rsz(4 * (Et + Gt)) + rsz(Et + Gt) + rsz(Ct);  // fl, fs, cdt
-    total += sz<double>(8 * (size_t)D.nblk) + sz<DState>(n) + sz<DRecord>(EBB_REC_CAP);
+    total += sz<double>(8 * (size_t)D.nblk) + sz<double>(10 * EBB_STEP_PARTS * (size_t)n) + sz<DState>(n) + sz<DRecord>(EBB_REC_CAP);
     total += 4 * sz<int32_t>(Ct) + 3 * rsz(Ct) + (D.any_mms ? rsz(4 * Ct) : 0);
     total += 2 * sz<int32_t>(MJ * Cs) + 3 * rsz(2 * MJ * Cs);
     total += split ? rsz(2 * MJ * Cs) + rsz(MJ * Cs) : 0;  // per-slot edge normal and length
@@ -557,6 +557,7 @@ int assemble(ebb_solver *s, std::vector<InstLayout> &Ls, int32_t precision, std:
     A.fs = takeR(Et + Gt);
     A.cdt = takeR(Ct);
     A.red = ar.take<double>(8 * (size_t)nblk);
+    A.endp = ar.take<double>(10 * EBB_STEP_PARTS * (size_t)n);
     A.st = ar.take<DState>(n);
     A.rec = ar.take<DRecord>(EBB_REC_CAP);
     A.R = A.aux;
@@ -579,6 +580,11 @@ int assemble(ebb_solver *s, std::vector<InstLayout> &Ls, int32_t precision, std:
              within(en, 2.0);
     M.n_inst = n;
     M.n_upd_blocks = nblk;
+    M.max_inst_blocks = nblk;
+    if (n > 1) {
+        M.max_inst_blocks = 0;
+        for (int k = 0; k < n; k++) M.max_inst_blocks = std::max(M.max_inst_blocks, inst_blk[k + 1] - inst_blk[k]);
+    }
     auto up = [&](auto *dst, const auto &v) {
         if (!v.empty()) cudaMemcpyAsync((void *)dst, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, s->stream);
         return dst;

@@ -21,6 +21,7 @@
 #define EBB_NOERR 0xFFFFFFFFFFFFFFFFull
 #define EBB_REC_CAP 4096
 #define EBB_RED_THREADS 256
+#define EBB_STEP_PARTS 16  // blocks of the step epilogue per instance, at most
 
 // real-valued mesh arrays, in the arithmetic type of a precision form
 struct DGeo {
@@ -50,6 +51,7 @@ struct DMesh {
     // batched arena of n_inst independent instances (all null when n_inst == 1):
     int32_t n_inst;
     int32_t n_upd_blocks;              // k_update grid size
+    int32_t max_inst_blocks;           // most k_update blocks of one instance
     const int32_t *cell_inst;          // instance of each interior cell
     const int32_t *blk_first, *blk_end, *blk_inst;  // k_update block -> cell range, instance
     const int32_t *inst_c0;            // n_inst+1 interior-cell offsets
@@ -97,21 +99,31 @@ struct DState {
     int64_t resid_min_iter;            // iteration of the smallest density residual so far
     double resid_min;                  // that residual
     ebbdf::df dtw, dt_half_w;          // double-float copies (the df path's stage states)
+    uint32_t end_count;                // parts of the step epilogue that have finished
 };
+
+// parts the step epilogue sums `rows` block partial sums in: one up to 256 rows, where a
+// thread adds 8 of them; 16 from 3,841 on, where it adds 8 of every 256
+EBB_DF_HD int step_parts(int rows)
+{
+    const int p = (rows + 255) / 256;
+    return p < 1 ? 1 : (p > EBB_STEP_PARTS ? EBB_STEP_PARTS : p);
+}
 
 // dt and what is derived from it: the halves and sixths of the RK stages and their FP32
 // (split path) and double-float (df path) copies
-EBB_DF_HD void set_step(DState &h, double dt)
+EBB_DF_HD void set_step(DState &h, double dt, double half, double sixth)
 {
     h.dt = dt;
-    h.dt_half = dt / 2.0;
-    h.dt_sixth = dt / 6.0;
+    h.dt_half = half;
+    h.dt_sixth = sixth;
     h.dtf = (float)dt;
     h.dt_half_f = (float)h.dt_half;
     h.dt_sixth_f = (float)h.dt_sixth;
     h.dtw = ebbdf::df(dt);
     h.dt_half_w = ebbdf::df(h.dt_half);
 }
+EBB_DF_HD void set_step(DState &h, double dt) { set_step(h, dt, dt / 2.0, dt / 6.0); }
 
 // record layout matches ebb_step_record
 struct DRecord {
@@ -139,6 +151,7 @@ struct DArrays {
     void *face, *grad, *fl, *fs, *cdt, *R;
     void *lim;            // T[8] per cell (lim[k][0], lim[k][1]) when exported, else null
     double *red;          // per-block partial sums (8 per block)
+    double *endp;         // the step epilogue's partial sums (10 per part, 16 parts per instance)
     DState *st;
     DRecord *rec;
 };
