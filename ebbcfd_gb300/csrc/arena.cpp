@@ -135,7 +135,6 @@ int build_instance(const ebb_mesh *mesh, const ebb_config *cfg, InstLayout &L, s
     L.snd.assign(2 * MJ * C, 0);
     L.sfd.assign(2 * MJ * C, 0);
     L.eslot.resize(2 * Eint);
-    L.ecell.resize(2 * Eint);
     L.eref.resize(Eint);
     L.en.resize(2 * Eint);
     L.elen.resize(Eint);
@@ -205,8 +204,6 @@ int build_instance(const ebb_mesh *mesh, const ebb_config *cfg, InstLayout &L, s
     }
     for (int64_t k = 0; k < Eint; k++) {
         const int32_t e2 = iedges[k];
-        L.ecell[2 * k] = inv[t.e_cell0[e2]];
-        L.ecell[2 * k + 1] = inv[t.e_cell1[e2]];
         L.en[2 * k] = t.e_nx[e2];
         L.en[2 * k + 1] = t.e_ny[e2];
         L.elen[k] = t.e_len[e2];
@@ -377,9 +374,8 @@ size_t bytes_of(const Dims &D, int32_t precision)
     total += sz<double>(8 * (size_t)D.nblk) + sz<double>(10 * EBB_STEP_PARTS * (size_t)n) + sz<DState>(n) + sz<DRecord>(EBB_REC_CAP);
     total += 4 * sz<int32_t>(Ct) + 3 * rsz(Ct) + (D.any_mms ? rsz(4 * Ct) : 0);
     total += 2 * sz<int32_t>(MJ * Cs) + 3 * rsz(2 * MJ * Cs);
-    total += split ? rsz(2 * MJ * Cs) + rsz(MJ * Cs) : 0;  // per-slot edge normal and length
-    total += 2 * sz<int32_t>(2 * Et) + rsz(2 * Et) + rsz(Et) + sz<int32_t>(Et);
-    total += 4 * sz<int32_t>(Gt) + rsz(2 * Gt) + rsz(Gt) + 4 * rsz(4 * Gt);
+    total += sz<int32_t>(2 * Et) + rsz(2 * (Et + Gt)) + rsz(Et + Gt) + sz<int32_t>(Et);
+    total += 4 * sz<int32_t>(Gt) + 4 * rsz(4 * Gt);
     total += sz<int32_t>(D.nforce + 1) + sz<int32_t>(n + 1);
     total += 2 * sz<double>(4 * Ct);  // host-order staging, device-order scratch
     if (n > 1) total += sz<int32_t>(Ct) + 3 * sz<int32_t>(D.nblk) + 2 * sz<int32_t>(n + 1) + sz<double>(n) + sz<float>(n);
@@ -437,7 +433,7 @@ int assemble(ebb_solver *s, std::vector<InstLayout> &Ls, int32_t precision, std:
     std::vector<int32_t> nedge(Ct), cellref(Ct), snbr(MJ * Cs, 0), sedge(MJ * Cs, 0);
     std::vector<double> nia(Ct), perim(Ct), d(Ct), src(any_mms ? 4 * Ct : 0);
     std::vector<double> sgm(2 * MJ * Cs, 0), snd(2 * MJ * Cs, 0), sfd(2 * MJ * Cs, 0);
-    std::vector<int32_t> eslot(2 * Et), ecell(2 * Et), eref(Et);
+    std::vector<int32_t> eslot(2 * Et), eref(Et);
     std::vector<double> en(2 * Et), elen(Et);
     std::vector<int32_t> bcell(Gt), bslot(Gt), btype(Gt), bref(Gt);
     std::vector<double> bn(2 * Gt), blen(Gt), brefl(4 * Gt), bdata(4 * Gt), bdq(4 * Gt), bdmid(4 * Gt);
@@ -488,8 +484,6 @@ int assemble(ebb_solver *s, std::vector<InstLayout> &Ls, int32_t precision, std:
         for (int64_t x = 0; x < L.Eint; x++) {
             eslot[2 * (e0 + x)] = gslot(L.eslot[2 * x]);
             eslot[2 * (e0 + x) + 1] = gslot(L.eslot[2 * x + 1]);
-            ecell[2 * (e0 + x)] = gcell(L.ecell[2 * x]);
-            ecell[2 * (e0 + x) + 1] = gcell(L.ecell[2 * x + 1]);
             en[2 * (e0 + x)] = L.en[2 * x];
             en[2 * (e0 + x) + 1] = L.en[2 * x + 1];
             elen[e0 + x] = L.elen[x];
@@ -580,6 +574,7 @@ int assemble(ebb_solver *s, std::vector<InstLayout> &Ls, int32_t precision, std:
              within(en, 2.0);
     M.n_inst = n;
     M.n_upd_blocks = nblk;
+    M.speeds = 1;
     M.max_inst_blocks = nblk;
     if (n > 1) {
         M.max_inst_blocks = 0;
@@ -623,32 +618,19 @@ int assemble(ebb_solver *s, std::vector<InstLayout> &Ls, int32_t precision, std:
     M.g.s_nd = upR(snd);
     M.g.s_fd = upR(sfd);
     M.e_slot = up(ar.take<int32_t>(2 * Et), eslot);
-    M.e_cell = up(ar.take<int32_t>(2 * Et), ecell);
+    // one array each: the split update reads the normals and lengths of a cell's edges
+    // by flux index, boundary edges included
+    en.insert(en.end(), bn.begin(), bn.end());
+    elen.insert(elen.end(), blen.begin(), blen.end());
     M.g.e_n = upR(en);
     M.g.e_len = upR(elen);
-    if (split) {  // per-slot copies for the split update's freestream correction
-        std::vector<double> sen(2 * MJ * Cs, 0.0), selen(MJ * Cs, 0.0);
-        for (int64_t i = 0; i < Ct; i++)
-            for (int j = 0; j < nedge[i]; j++) {
-                const int64_t gs = (int64_t)j * Cs + i;
-                const int64_t f = sedge[gs] & 0x7fffffff;
-                const bool in = f < Et;
-                sen[2 * gs] = in ? en[2 * f] : bn[2 * (f - Et)];
-                sen[2 * gs + 1] = in ? en[2 * f + 1] : bn[2 * (f - Et) + 1];
-                selen[gs] = in ? elen[f] : blen[f - Et];
-            }
-        M.g.s_en = upR(sen);
-        M.g.s_elen = upR(selen);
-    } else {
-        M.g.s_en = M.g.s_elen = nullptr;
-    }
+    M.g.b_n = static_cast<const char *>(M.g.e_n) + 2 * Et * (split ? sizeof(float) : sizeof(double));
+    M.g.b_len = static_cast<const char *>(M.g.e_len) + Et * (split ? sizeof(float) : sizeof(double));
     M.e_ref = up(ar.take<int32_t>(Et), eref);
     M.b_cell = up(ar.take<int32_t>(Gt), bcell);
     M.b_slot = up(ar.take<int32_t>(Gt), bslot);
     M.b_type = up(ar.take<int32_t>(Gt), btype);
     M.b_ref = up(ar.take<int32_t>(Gt), bref);
-    M.g.b_n = upR(bn);
-    M.g.b_len = upR(blen);
     M.g.b_refl = upR(brefl);
     M.g.b_data = upR(bdata);
     M.g.b_dq = upR(bdq);

@@ -9,7 +9,7 @@
 //           nbr int32, edge int32 (bit 31 = fluxMultiplier -1), gm T[2] (gradMat column),
 //           nd T[2] (neighbour centroid - centroid), fd T[2] (edge midpoint - centroid),
 //           face T[4] (reconstructed face state)
-//   edges   slot int32[2], cell int32[2], n T[2], len T; fluxes fl T[4] (len*F) and fs T
+//   edges   slot int32[2], n T[2], len T (boundary edges after them); fluxes fl T[4] (len*F) and fs T
 //           (len*sMax) for interior edges then boundary edges
 //   cells   nedge int32, neg_inv_area, perim, d, src T[4] (manufactured source)
 // All geometry is computed on the host in FP64; the split path stores FP32 copies.
@@ -28,20 +28,19 @@ struct DGeo {
     const void *s_gm, *s_nd, *s_fd;             // T[2] per slot
     const void *neg_inv_area, *perim, *dlen;     // T per cell
     const void *src;                             // T[4] per cell or null
-    const void *e_n, *e_len;                     // T[2], T per interior edge
-    const void *s_en, *s_elen;                   // split path: T[2], T per slot, a copy of
-                                                 // the slot's edge normal and length
-    const void *b_n, *b_len;                     // T[2], T per boundary edge
+    const void *e_n, *e_len;                     // T[2], T per edge, interior ones first
+    const void *b_n, *b_len;                     // the boundary edges' part of them
     const void *b_refl, *b_data, *b_dq, *b_dmid; // T[4] per boundary edge
 };
 
 struct DMesh {
     int32_t C, G, Cs, Eint, maxJ;
     int32_t uniform;                   // every interior cell has exactly maxJ edges
+    int32_t rev, speeds;               // of a launch: blocks in descending order; edge speeds (fs) wanted
     int32_t soft;                      // gradient weights, offsets and normals are zero or of ordinary size (see arena.cpp)
     const int32_t *nedge;
     const int32_t *s_nbr, *s_edge;
-    const int32_t *e_slot, *e_cell;    // int2 per interior edge
+    const int32_t *e_slot;             // int2 per interior edge
     const int32_t *b_cell, *b_slot, *b_type;
     const int32_t *e_ref, *b_ref;      // reference edge ids (error reports)
     const int32_t *cell_ref;           // reference cell id per device cell

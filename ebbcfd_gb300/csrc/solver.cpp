@@ -118,12 +118,20 @@ inline double bitsd(unsigned long long u)
     return v;
 }
 
+// One stage's three kernels, each through the mesh in the other direction than the one
+// before it (`odd`: the stage's number in its step is odd).
 template <typename T>
-int run_stage_t(ebb_solver *s, int stage, T *qin, T *qout, int limit, int dt_update, int need_dt, int final_stage)
+int run_stage_t(ebb_solver *s, int stage, T *qin, T *qout, int limit, int dt_update, int need_dt, int final_stage,
+                int odd = 0)
 {
-    CKL(launch_cell<T>(s->M, s->P, s->A, qin, limit, s->stream));
-    CKL(launch_flux<T>(s->M, s->P, s->A, qin, s->stream));
-    CKL(launch_update<T>(s->M, s->P, s->A, stage, qin, qout, dt_update, need_dt, final_stage, s->stream));
+    DMesh M = s->M;
+    M.speeds = need_dt || (s->P.local_ts && dt_update);
+    M.rev = odd;
+    CKL(launch_cell<T>(M, s->P, s->A, qin, limit, s->stream));
+    M.rev = !odd;
+    CKL(launch_flux<T>(M, s->P, s->A, qin, s->stream));
+    M.rev = odd;
+    CKL(launch_update<T>(M, s->P, s->A, stage, qin, qout, dt_update, need_dt, final_stage, s->stream));
     return EBB_OK;
 }
 
@@ -141,17 +149,17 @@ template <typename T> int integrator_stages_t(ebb_solver *s)
         break;
     case EBB_INT_RK2:
         if ((r = run_stage_t<T>(s, ST_RK2_1, q1, qs, 1, 1, 0, 0))) break;
-        r = run_stage_t<T>(s, ST_RK2_2, qs, q1, ms, 0, 1, 1);
+        r = run_stage_t<T>(s, ST_RK2_2, qs, q1, ms, 0, 1, 1, 1);
         break;
     case EBB_INT_RK2_TVD:
         if ((r = run_stage_t<T>(s, ST_TVD_1, q1, qs, 1, lts, 0, 0))) break;
-        r = run_stage_t<T>(s, ST_TVD_2, qs, q1, 0, !lts, 1, 1);
+        r = run_stage_t<T>(s, ST_TVD_2, qs, q1, 0, !lts, 1, 1, 1);
         break;
     case EBB_INT_RK4:
         if ((r = run_stage_t<T>(s, ST_RK4_1, q1, qs, 1, 1, 0, 0))) break;
-        if ((r = run_stage_t<T>(s, ST_RK4_2, qs, qs, ms, 0, 0, 0))) break;
+        if ((r = run_stage_t<T>(s, ST_RK4_2, qs, qs, ms, 0, 0, 0, 1))) break;
         if ((r = run_stage_t<T>(s, ST_RK4_3, qs, qs, ms, 0, 0, 0))) break;
-        r = run_stage_t<T>(s, ST_RK4_4, qs, q1, ms, 0, 1, 1);
+        r = run_stage_t<T>(s, ST_RK4_4, qs, q1, ms, 0, 1, 1, 1);
         break;
     default:
         r = fail(s, EBB_ERR_CONFIG, "unknown integrator");

@@ -19,7 +19,7 @@ struct InstLayout {
     int maxJ = 0;
     double mu = 0;
     bool any_visc_wall = false;
-    std::vector<int32_t> perm, cellref, nedge, snbr, sedge, eslot, ecell, eref;
+    std::vector<int32_t> perm, cellref, nedge, snbr, sedge, eslot, eref;
     std::vector<int32_t> bcell, bslot, btype, bref, force, ref_nedge;
     std::vector<int64_t> ref_face_slot;
     std::vector<double> nia, perim, d, src, sgm, snd, sfd, en, elen, bn, blen, brefl, bdata, bdq, bdmid, grad, q;

@@ -14,6 +14,7 @@
 // split_inv k_cell: 64x12 30.9 us, 64x16 27.4 us, 128x6 31.9 us, 128x8 27.8 us, 128x10 32.5 us, 256x3 32.8 us, 256x4 27.8 us
 // split_inv k_flux: 64x16 27.0 us, 64x20 26.9 us, 128x8 23.4 us, 128x10 22.3 us, 128x12 20.3 us, 256x4 25.4 us, 256x6 20.9 us
 // split_inv k_update: 256x4 32.3 us, 256x6 30.0 us, 256x8 28.9 us, 512x2 35.3 us, 512x3 30.6 us, 512x4 29.3 us
+// split_inv k_update since (500,000 cells, by hand): 256x4 11.6 us, 256x5 11.5 us, 256x6 14.0 us, 256x7 15.1 us
 // update block size 256 (summed best update times: 256: 987.6 us, 512: 1063.9 us)
 #pragma once
 #ifndef EBB_CELL_TB_F
@@ -77,5 +78,5 @@
 #define EBB_FLUX_MINB_FI 12
 #endif
 #ifndef EBB_UPD_MINB_FI
-#define EBB_UPD_MINB_FI 8
+#define EBB_UPD_MINB_FI 5
 #endif
