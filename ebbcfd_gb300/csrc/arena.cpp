@@ -571,7 +571,7 @@ int assemble(ebb_solver *s, std::vector<InstLayout> &Ls, int32_t precision, std:
         });
     };
     M.soft = precision == EBB_PREC_FP64 && within(sgm, 0x1p100) && within(snd, 0x1p20) && within(sfd, 0x1p20) &&
-             within(en, 2.0);
+             within(en, 2.0) && within(bn, 2.0);
     M.n_inst = n;
     M.n_upd_blocks = nblk;
     M.speeds = 1;
@@ -684,6 +684,8 @@ int assemble(ebb_solver *s, std::vector<InstLayout> &Ls, int32_t precision, std:
     P.m1gP = -1.0 + P.gP;
     P.p43mgP = (4.0 / 3.0) - P.gP;
     P.omgP = 1.0 - P.gP;
+    if (c0.viscosity || visc_wall)  // the viscous flux's constants, for the integer-pipe products
+        M.soft = M.soft && P.gP != 0 && within({P.gP, P.c43gP, P.m1gP, P.p43mgP, P.omgP}, 0x1p100);
     P.gPw = P.gP;
     P.c43gPw = P.c43gP;
     P.m1gPw = P.m1gP;

@@ -4,9 +4,10 @@
 //
 // The plain FP64 flux kernel is bound by the FP64 pipe (a warp instruction every 64
 // cycles of a scheduler: ~440 of them per face kept it 85% busy with 8% of the issue
-// slots used).  Here about 130 remain per face, additions mostly, beside ~6,500 other
-// instructions: the pipe is 64% busy, the integer pipe 53%.  Per launch, 400,000 plate
-// cells: 241 us, 548 us with device_math.cuh; 200,000 triangles (Rusanov): 56 and 136 us.
+// slots used).  Here about 125 remain per face, additions mostly, beside ~6,000 other
+// instructions: the pipe is 67% busy, the integer pipe 54%.  Per launch, 400,000 plate
+// cells: 200 us, 548 us with device_math.cuh; 200,000 triangles (Rusanov): 41 and 136 us
+// (both with the boundary faces' part, which used to run last and alone: k_flux).
 // Three things keep the integer part from costing what it saves:
 //  * code size: as straight-line code a quarter of the warps' time went to instruction
 //    fetches (287 us).  The two sides of a face, the two directions of the viscous
@@ -15,8 +16,8 @@
 //    which takes it as a fused multiply-add by 0.5 (one rounding, the same), and the
 //    flux itself is returned doubled (the caller halves the edge length instead);
 //  * range checks: products need normal operands and results.  With the face states in
-//    2^+-60 (density) and 2^+-100 or zero, normals in [2^-100, 2] and (viscous) gradients
-//    and viscosity in 2^+-100, every operand below stays a normal number or an exact
+//    2^+-60 (density) and 2^+-100 or zero, normals in [2^-100, 2] and (viscous) gradients,
+//    viscosity and Prandtl-number terms in 2^+-100, every operand below stays a normal number or an exact
 //    zero: a sum of two terms is zero or at least the smaller one's last place, so each
 //    sum lowers a bound by 53 binary digits at most, and no chain of products here comes
 //    below 2^-960 or above 2^960.  Only the wave strengths C1, C2, which multiply four
@@ -40,6 +41,14 @@ template <int GROUP> __device__ __forceinline__ double sm(double a, double b)
 {
     if constexpr ((EBB_SOFT_GROUPS >> GROUP) & 1)
         return ebbsoft::mul(a, b);
+    else
+        return a * b;
+}
+// the same for an a that is not zero
+template <int GROUP> __device__ __forceinline__ double smn(double a, double b)
+{
+    if constexpr ((EBB_SOFT_GROUPS >> GROUP) & 1)
+        return ebbsoft::mul<true>(a, b);
     else
         return a * b;
 }
@@ -70,14 +79,14 @@ __device__ __forceinline__ void soft_side(const double q[4], double nx, double n
     S.u = u;
     S.v = v;
     const double uu = sm<G>(u, u), vv = sm<G>(v, v);
-    S.rv0 = sm<G>(rho, u);
-    S.rv1 = sm<G>(rho, v);
-    const double p = sm<G>(K<double>::gm1, fma(-0.5, sm<G>(rho, uu + vv), e));
+    S.rv0 = smn<G>(rho, u);
+    S.rv1 = smn<G>(rho, v);
+    const double p = smn<G>(K<double>::gm1, fma(-0.5, smn<G>(rho, uu + vv), e));
     S.p = p;
     const double pe = p + e;
     if (H) S.h = ebbsoft::div(pe, S.R);
-    const double f1 = p + sm<G>(rho, uu), f2 = sm<G>(S.rv0, v), f3 = sm<G>(u, pe);
-    const double h2 = p + sm<G>(rho, vv), h3 = sm<G>(v, pe);
+    const double f1 = p + smn<G>(rho, uu), f2 = sm<G>(S.rv0, v), f3 = sm<G>(u, pe);
+    const double h2 = p + smn<G>(rho, vv), h3 = sm<G>(v, pe);
     f[0] = sm<C>(S.rv0, nx) + sm<C>(S.rv1, ny);
     f[1] = sm<C>(f1, nx) + sm<C>(f2, ny);
     f[2] = sm<C>(f2, nx) + sm<C>(h2, ny);
@@ -110,18 +119,17 @@ __device__ __forceinline__ void soft_sides(const double qL[4], const double qR[4
 // the entropy-fixed wave speeds |u + a|, |u - a|, |u| (l1, l2, l3)
 __device__ __forceinline__ void soft_speeds(double u, double a, double &l1, double &l2, double &l3, bool &bad)
 {
-    const double eps = 0.01 * a;
+    const double eps = ebbsoft::mul<true>(0.01, a);
     l1 = fabs(u + a);
     l2 = fabs(u - a);
     l3 = fabs(u);
     if (l1 < eps || l2 < eps || l3 < eps) {
-        const double e2 = eps * eps;
-        const double d = 2.0 * eps;
+        const double e2 = ebbsoft::mul<true>(eps, eps), d = ebbsoft::twice(eps);
         bad |= !ebbsoft::divisor_ok(d);
         const ebbsoft::Recip R = ebbsoft::recip(d);
 #pragma unroll 1
         for (int r = 0; r < 3; r++) {
-            const double l = l1 < eps ? ebbsoft::div(e2 + l1 * l1, R) : l1;
+            const double l = l1 < eps ? ebbsoft::div(e2 + ebbsoft::mul(l1, l1), R) : l1;
             l1 = l2;
             l2 = l3;
             l3 = l;
@@ -139,12 +147,13 @@ __device__ __forceinline__ void roe_flux2_soft(const double qL[4], const double 
     soft_sides<true>(qL, qR, nx, ny, A, B, fs, bad);
     const double di = ebbsoft::root(ebbsoft::div(B.rho, A.R), bad);
     const double d1 = soft_ratio(1.0, 1.0 + di, bad);
-    const double vel0 = sm<M>(sm<M>(di, B.u) + A.u, d1);
-    const double vel1 = sm<M>(sm<M>(di, B.v) + A.v, d1);
+    const double vel0 = smn<M>(d1, smn<M>(di, B.u) + A.u);
+    const double vel1 = smn<M>(d1, smn<M>(di, B.v) + A.v);
     const double u = sm<M>(vel0, nx) + sm<M>(vel1, ny);
-    const double h = sm<M>(sm<M>(di, B.h) + A.h, d1);
+    const double h = smn<M>(d1, smn<M>(di, B.h) + A.h);
     const double vv = sm<M>(vel0, vel0) + sm<M>(vel1, vel1);
-    const double a = ebbsoft::root(K<double>::gm1d * fma(-0.5, vv, h), bad);
+    const double a = ebbsoft::root(smn<M>(K<double>::gm1d, fma(-0.5, vv, h)), bad);
+    bad |= !ebbsoft::divisor_ok(a);
     const double dRV0 = B.rv0 - A.rv0, dRV1 = B.rv1 - A.rv1;
     const double dRho = qR[0] - qL[0], dRhoE = qR[3] - qL[3];
     double l1, l2, l3;
@@ -153,18 +162,17 @@ __device__ __forceinline__ void roe_flux2_soft(const double qL[4], const double 
     // s1 - l3 and twice s2; G1's first term doubled
     const double sl = fma(0.5, l1 + l2, -l3), s2 = l1 - l2;
     const double qq = ebbsoft::root(vv, bad);
-    const double G1 = sm<W>(K<double>::gm1, fma(0.5, sm<W>(sm<W>(qq, qq), dRho), -(sm<W>(vel0, dRV0) + sm<W>(vel1, dRV1))) + dRhoE);
+    const double G1 = smn<W>(K<double>::gm1, fma(0.5, sm<W>(sm<W>(qq, qq), dRho), -(sm<W>(vel0, dRV0) + sm<W>(vel1, dRV1))) + dRhoE);
     const double G2 = sm<W>(-u, dRho) + (sm<W>(dRV0, nx) + sm<W>(dRV1, ny));
-    bad |= !ebbsoft::divisor_ok(a);
     const ebbsoft::Recip R = ebbsoft::recip(a);
-    const double C1 = fma(0.5, ebbsoft::div(G2, R) * s2, soft_ratio(G1, a * a, bad) * sl);
+    const double C1 = fma(0.5, ebbsoft::div(G2, R) * s2, soft_ratio(G1, ebbsoft::mul<true>(a, a), bad) * sl);
     const double C2 = fma(0.5, ebbsoft::div(G1, R) * s2, sl * G2);
     ebbsoft::check<400>(C1, bad);
     ebbsoft::check<400>(C2, bad);
-    out[0] = fs[0] - (sm<W>(l3, dRho) + C1);
-    out[1] = fs[1] - (sm<W>(l3, dRV0) + sm<W>(C1, vel0) + sm<W>(C2, nx));
-    out[2] = fs[2] - (sm<W>(l3, dRV1) + sm<W>(C1, vel1) + sm<W>(C2, ny));
-    out[3] = fs[3] - (sm<W>(l3, dRhoE) + sm<W>(C1, h) + sm<W>(C2, u));
+    out[0] = fs[0] - (smn<W>(l3, dRho) + C1);
+    out[1] = fs[1] - (smn<W>(l3, dRV0) + sm<W>(C1, vel0) + sm<W>(C2, nx));
+    out[2] = fs[2] - (smn<W>(l3, dRV1) + sm<W>(C1, vel1) + sm<W>(C2, ny));
+    out[3] = fs[3] - (smn<W>(l3, dRhoE) + sm<W>(C1, h) + sm<W>(C2, u));
 }
 
 // twice the Rusanov flux (source/flux.d:66-141, the reduced form of rusanov_flux)
@@ -175,23 +183,23 @@ __device__ __forceinline__ void rusanov_flux2_soft(const double qL[4], const dou
     SoftSide A, B;
     double fs[4];
     soft_sides<false>(qL, qR, nx, ny, A, B, fs, bad);
-    const double rho = ebbsoft::root(sm<M>(A.rho, B.rho), bad);
+    const double rho = ebbsoft::root(smn<M>(A.rho, B.rho), bad);
     const double sL = ebbsoft::root(A.rho, bad), sR = ebbsoft::root(B.rho, bad);
     const ebbsoft::Recip S = ebbsoft::recip(sL + sR);
-    const double vel0 = ebbsoft::div(sm<M>(sL, A.u) + sm<M>(sR, B.u), S);
-    const double vel1 = ebbsoft::div(sm<M>(sL, A.v) + sm<M>(sR, B.v), S);
+    const double vel0 = ebbsoft::div(smn<M>(sL, A.u) + smn<M>(sR, B.u), S);
+    const double vel1 = ebbsoft::div(smn<M>(sL, A.v) + smn<M>(sR, B.v), S);
     const double u = sm<M>(vel0, nx) + sm<M>(vel1, ny);
-    const double p = ebbsoft::div(sm<M>(sL, A.p) + sm<M>(sR, B.p), S);
-    const double a = ebbsoft::root(K<double>::g * ebbsoft::div(p, ebbsoft::recip(rho)), bad);
+    const double p = ebbsoft::div(smn<M>(sL, A.p) + smn<M>(sR, B.p), S);
+    const double a = ebbsoft::root(smn<M>(K<double>::g, ebbsoft::div(p, ebbsoft::recip(rho))), bad);
     bad |= !ebbsoft::divisor_ok(a);
     double l1, l2, l3;
     soft_speeds(u, a, l1, l2, l3, bad);
     const double s = max4(l1, l2, l3, l3);
     sMax = s;
-    out[0] = fs[0] - sm<W>(s, qR[0] - qL[0]);
-    out[1] = fs[1] - sm<W>(s, B.rv0 - A.rv0);
-    out[2] = fs[2] - sm<W>(s, B.rv1 - A.rv1);
-    out[3] = fs[3] - sm<W>(s, qR[3] - qL[3]);
+    out[0] = fs[0] - smn<W>(s, qR[0] - qL[0]);
+    out[1] = fs[1] - smn<W>(s, B.rv0 - A.rv0);
+    out[2] = fs[2] - smn<W>(s, B.rv1 - A.rv1);
+    out[3] = fs[3] - smn<W>(s, qR[3] - qL[3]);
 }
 
 __device__ __forceinline__ void inviscid_flux2_soft(int kind, const double qL[4], const double qR[4], double nx, double ny,
@@ -203,9 +211,9 @@ __device__ __forceinline__ void inviscid_flux2_soft(int kind, const double qL[4]
         rusanov_flux2_soft(qL, qR, nx, ny, out, sMax, bad);
 }
 
-// Twice the viscous flux (source/flux.d:28-64) of twice the face state q and gradients dq:
-// the quotients by the density do not see the factor, the fluxes are linear in dq, and mu
-// over half the density is 2 mu over it.  Component 0 is a signed zero (zero_dot) and
+// Twice the viscous flux (source/flux.d:28-64) of the face state q and gradients dq, or of
+// their halves: the quotients by the density do not see a factor in q, mu over the density
+// takes it on, and the fluxes are linear in dq.  Component 0 is a signed zero (zero_dot) and
 // left to the caller.  Directions x and y run the same loop body: a matrix entry of the
 // second is the first's with u and v (and the two coefficients of a pair) exchanged.
 __device__ __forceinline__ void diffusive_flux2_soft(const ViscConst<double> &vc, double mu, const double q[4],
@@ -220,40 +228,50 @@ __device__ __forceinline__ void diffusive_flux2_soft(const ViscConst<double> &vc
     }
     const ebbsoft::Recip R = ebbsoft::recip(q[0]);
     const double u = ebbsoft::div(q[1], R), v = ebbsoft::div(q[2], R), E = ebbsoft::div(q[3], R);
-    const double s = ebbsoft::div(2.0 * mu, R);
-    const double c43 = -4.0 / 3.0, p43 = 4.0 / 3.0, p23 = 2.0 / 3.0, m23 = -2.0 / 3.0, c231 = 2.0 / 3.0 - 1.0;
-    const double uu = sm<M>(u, u), vv = sm<M>(v, v), gE = sm<M>(vc.gP, E);
-    const double b30 = sm<M>(s, sm<M>(sm<M>(c231, u), v));
-    const double sp43 = sm<M>(s, p43), sm23 = sm<M>(s, m23), sgP = sm<M>(s, vc.gP);
+    bad |= (ebbsoft::hi_of(mu) & ebbsoft::kExp) == 0u;
+    const double s = ebbsoft::div(ebbsoft::twice(mu), R);
+    const double c43 = -4.0 / 3.0, p43 = 4.0 / 3.0, m23 = -2.0 / 3.0, c231 = 2.0 / 3.0 - 1.0;
+    const double uu = sm<M>(u, u), vv = sm<M>(v, v), gE = smn<M>(vc.gP, E);
+    const double b30 = smn<M>(s, sm<M>(smn<M>(c231, u), v));
+    const double sp43 = smn<M>(s, p43), sm23 = smn<M>(s, m23), sgP = smn<M>(s, vc.gP);
+    const double su = smn<M>(s, u), sv = smn<M>(s, v), tu = smn<M>(s, smn<M>(m23, u)), tv = smn<M>(s, smn<M>(m23, v));
     // row 2 of the x matrices is row 1 of the y ones
-    const double G12 = (zero_plus(sm<S>(sm<M>(s, -v), dq[0][0])) + sm<S>(s, dq[2][0])) +
-                       (zero_plus(sm<S>(sm<M>(s, -u), dq[0][1])) + sm<S>(s, dq[1][1]));
+    const double G12 = (zero_plus(sm<S>(-sv, dq[0][0])) + smn<S>(s, dq[2][0])) +
+                       (zero_plus(sm<S>(-su, dq[0][1])) + smn<S>(s, dq[1][1]));
     double Gn[4];  // G0_1, G0_3, G1_2, G1_3
     double z0 = dq[0][0], z1 = dq[1][0], z2 = dq[2][0], z3 = dq[3][0];
     double w0 = dq[0][1], w1 = dq[1][1], w2 = dq[2][1], w3 = dq[3][1];
-    double zn = z1;                                         // normal-stress gradient
-    double U = u, V = v;                                    // velocity along and across
-    double tA = vc.c43gP, tB = vc.m1gP, kA = vc.p43mgP, kB = vc.omgP, eA = 1.0, eB = m23;
-#pragma unroll 1
-    for (int d = 0; d < 2; d++) {
-        Gn[0] = Gn[2];
-        Gn[1] = Gn[3];
-        Gn[2] = (zero_plus(sm<S>(sm<M>(s, sm<M>(c43, U)), z0)) + sm<S>(sp43, zn)) +
-                (zero_plus(sm<S>(sm<M>(s, sm<M>(p23, V)), w0)) + sm<S>(sm23, w2));
-        const double t = sm<M>(tA, uu) + sm<M>(tB, vv) - gE;
-        Gn[3] = (zero_plus(sm<S>(sm<M>(s, t), z0)) + sm<S>(sm<M>(s, sm<M>(kA, u)), z1) + sm<S>(sm<M>(s, sm<M>(kB, v)), z2) +
-                 sm<S>(sgP, z3)) +
-                (zero_plus(sm<S>(b30, w0)) + sm<S>(sm<M>(s, sm<M>(eA, v)), w1) + sm<S>(sm<M>(s, sm<M>(eB, u)), w2));
+    double zn = z1;                                // normal-stress gradient
+    double U = u, tV = -tv, tW = -tu;              // velocity along; s 2/3 times that across
+    double tA = vc.c43gP, tB = vc.m1gP, kA = vc.p43mgP, kB = vc.omgP, eA = sv, eB = tu;
+    auto next_direction = [&]() {
         zn = w2;
         double x = z0;
         z0 = w0, w0 = x;
         x = z1, z1 = w1, w1 = x;
         x = z2, z2 = w2, w2 = x;
         z3 = w3;
-        x = U, U = V, V = x;
+        U = v;
+        tV = tW;
         x = tA, tA = tB, tB = x;
         x = kA, kA = kB, kB = x;
-        x = eA, eA = eB, eB = x;
+        eA = tv;
+        eB = su;
+    };
+    auto rows = [&](double &n, double &e) {
+        n = (zero_plus(sm<S>(smn<M>(s, smn<M>(c43, U)), z0)) + smn<S>(sp43, zn)) +
+            (zero_plus(sm<S>(tV, w0)) + smn<S>(sm23, w2));
+        const double t = sm<M>(tA, uu) + sm<M>(tB, vv) - gE;
+        e = (zero_plus(sm<S>(smn<M>(s, t), z0)) + sm<S>(smn<M>(s, sm<M>(kA, u)), z1) +
+             sm<S>(smn<M>(s, sm<M>(kB, v)), z2) + smn<S>(sgP, z3)) +
+            (zero_plus(sm<S>(b30, w0)) + sm<S>(eA, w1) + sm<S>(eB, w2));
+    };
+#pragma unroll 1
+    for (int d = 0; d < 2; d++) {
+        Gn[0] = Gn[2];
+        Gn[1] = Gn[3];
+        rows(Gn[2], Gn[3]);
+        next_direction();
     }
     out[1] = sm<SG_OUT>(Gn[0], nx) + sm<SG_OUT>(G12, ny);
     out[2] = sm<SG_OUT>(G12, nx) + sm<SG_OUT>(Gn[2], ny);

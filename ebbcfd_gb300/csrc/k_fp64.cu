@@ -14,14 +14,6 @@ using namespace ebbdev;
 
 namespace {
 
-// sqrt(x) and a / b, on the integer pipe where the values allow it
-__device__ __forceinline__ double quick_root(double x)
-{
-    bool bad = false;
-    const double r = ebbsoft::root(x, bad);
-    return bad ? sqrt(x) : r;
-}
-
 // end of one runIntegrator iteration (app/solver.d:126-249).  blockIdx.y: the instance;
 // blockIdx.x: a part of its rows of block partial sums (step_parts of them, a function of
 // the instance's size alone, so that an instance sums in the same order in any arena).
@@ -99,7 +91,7 @@ template <typename T> __global__ void __launch_bounds__(EBB_RED_THREADS) k_step_
     const double dt = st->dynamic_dt ? __longlong_as_double((long long)st->newdt_bits) : st->dt;
     double x = 0.0;
     if (lane < 4)
-        x = ratio(quick_root((double)ncell * v), vs);
+        x = ratio(root((double)ncell * v), vs);
     else if (lane < 6)
         x = st->rot[2 * (lane - 4)] * fx + st->rot[2 * (lane - 4) + 1] * fy;
     else if (lane == 6)

@@ -342,6 +342,20 @@ template <typename T> __device__ __forceinline__ typename V2<T>::t lds2(const vo
 }
 template <typename T> __device__ __forceinline__ const T *ptr(const void *base) { return reinterpret_cast<const T *>(base); }
 
+// a / b and sqrt(x), FP64 on the integer pipe where the values allow it
+template <typename T> __device__ __forceinline__ T ratio(T a, T b) { return a / b; }
+template <> __device__ __forceinline__ double ratio<double>(double a, double b)
+{
+    return ebbdiv::div(a, ebbdiv::recip(b));
+}
+template <typename T> __device__ __forceinline__ T root(T x) { return dsqrt(x); }
+template <> __device__ __forceinline__ double root<double>(double x)
+{
+    bool bad = false;
+    const double r = ebbsoft::root(x, bad);
+    return bad ? sqrt(x) : r;
+}
+
 template <typename T>
 __device__ __forceinline__ void reflect(int type, const T *refl, T v0, T v1, T &o0, T &o1)
 {
@@ -369,7 +383,7 @@ __device__ void ghost_state(const DMesh &M, const DPhys &P, DState *st, int b, c
         break;
     case BC_INVWALL:
     case BC_SYMMETRY: {
-        T v0 = qi[1] / qi[0], v1 = qi[2] / qi[0], n0, n1;
+        T v0 = ratio(qi[1], qi[0]), v1 = ratio(qi[2], qi[0]), n0, n1;
         reflect(type, ptr<T>(M.g.b_refl) + 4 * (size_t)b, v0, v1, n0, n1);
         qn[0] = qi[0];
         qn[1] = qi[0] * n0;
@@ -384,18 +398,18 @@ __device__ void ghost_state(const DMesh &M, const DPhys &P, DState *st, int b, c
         qn[3] = qi[3];
         break;
     case BC_CONSTP: {
-        T rhop = qi[0], up = qi[1] / qi[0], vp = qi[2] / qi[0];
+        T rhop = qi[0], up = ratio(qi[1], qi[0]), vp = ratio(qi[2], qi[0]);
         T pp = pressure(qi);
-        T ap = dsqrt(G * (pp / rhop));
-        T Jp = up + (T(2.0) * ap) / (G - 1);
-        T Sp = pp / dpow(rhop, G);
+        T ap = root(G * ratio(pp, rhop));
+        T Jp = up + ratio(T(2.0) * ap, G - 1);
+        T Sp = ratio(pp, dpow(rhop, G));
         T pb = ptr<T>(M.g.b_data)[4 * (size_t)b];
-        T rhob = dpow(pb / Sp, T(1.0 / 1.4));
-        T ab = dsqrt(G * (pb / rhob));
-        T ub = Jp - (T(2.0) * ab) / (G - 1);
+        T rhob = dpow(ratio(pb, Sp), T(1.0 / 1.4));
+        T ab = root(G * ratio(pb, rhob));
+        T ub = Jp - ratio(T(2.0) * ab, G - 1);
         T vb = vp;
-        T mag = dsqrt(ub * ub + vb * vb);
-        T rEb = pb / (G - 1) + T(0.5) * rhob * (mag * mag);
+        T mag = root(ub * ub + vb * vb);
+        T rEb = ratio(pb, G - 1) + T(0.5) * rhob * (mag * mag);
         const typename V2<T>::t n = ld2<T>(M.g.b_n, b);
         T vpn = up * n.x + vp * n.y;
         T vbn = ub * n.x + vb * n.y;
@@ -1174,6 +1188,63 @@ template <typename T> __device__ __forceinline__ bool has_nan(const T F[4])
     return isnan(F[0]) || isnan(F[1]) || isnan(F[2]) || isnan(F[3]);
 }
 
+// The inviscid and viscous flux of a boundary face.  FP64: flux_soft.cuh's where the values
+// allow it.  A boundary block's latency is one face's: with device_math.cuh's ~450 FP64
+// instructions it was all of k_flux on small meshes (13.4 us on 1024 quads).
+template <typename T>
+__device__ __noinline__ void inviscid_plain(int kind, const T qL[4], const T qR[4], T nx, T ny, T F[4], T &sMax)
+{
+    inviscid_flux(kind, qL, qR, nx, ny, F, sMax);
+}
+template <typename T>
+__device__ __noinline__ void viscous_plain(const ViscConst<T> &vc, T mu, const T q[4], const T dq[4][2], T nx, T ny, T F[4])
+{
+    diffusive_flux(vc, mu, q, dq, nx, ny, F);
+}
+template <typename T>
+__device__ __forceinline__ void face_inviscid(const DMesh &M, int kind, const T qL[4], const T qR[4], T nx, T ny, T F[4],
+                                              T &sMax)
+{
+    if constexpr (is_fp64<T>) {
+        bool bad = !M.soft;
+        double X[4], s;
+        inviscid_flux2_soft(kind, qL, qR, nx, ny, X, s, bad);
+        if (bad) {
+            const double a[4] = {qL[0], qL[1], qL[2], qL[3]}, b[4] = {qR[0], qR[1], qR[2], qR[3]};
+            inviscid_plain<T>(kind, a, b, nx, ny, X, s);
+        }
+        sMax = s;
+#pragma unroll
+        for (int k = 0; k < 4; k++) F[k] = bad ? X[k] : 0.5 * X[k];
+    } else {
+        inviscid_flux(kind, qL, qR, nx, ny, F, sMax);
+    }
+}
+template <typename T>
+__device__ __forceinline__ void face_viscous(const DMesh &M, const ViscConst<T> &vc, T mu, const T q[4], const T dq[4][2],
+                                             T nx, T ny, T F[4])
+{
+    if constexpr (is_fp64<T>) {
+        bool bad = !M.soft;
+        ebbsoft::check<60>(q[0], bad);
+        bad |= !ebbsoft::divisor_ok(q[0]);
+#pragma unroll
+        for (int k = 1; k < 4; k++) ebbsoft::check<100>(q[k], bad);
+        double X[4];
+        diffusive_flux2_soft(vc, mu, q, dq, nx, ny, X, bad);
+        if (bad) {
+            const double a[4] = {q[0], q[1], q[2], q[3]};
+            const double g[4][2] = {{dq[0][0], dq[0][1]}, {dq[1][0], dq[1][1]}, {dq[2][0], dq[2][1]}, {dq[3][0], dq[3][1]}};
+            viscous_plain<T>(vc, mu, a, g, nx, ny, X);
+        }
+        F[0] = zero_dot(nx, ny);
+#pragma unroll
+        for (int k = 1; k < 4; k++) F[k] = bad ? X[k] : 0.5 * X[k];
+    } else {
+        diffusive_flux(vc, mu, q, dq, nx, ny, F);
+    }
+}
+
 template <typename T>
 __device__ void boundary_flux(const DMesh &M, const DPhys &P, const DArrays &A, const T *qin, int b)
 {
@@ -1197,7 +1268,7 @@ __device__ void boundary_flux(const DMesh &M, const DPhys &P, const DArrays &A, 
     case BC_FULLSTATE: {
         T qR[4];
         ld4(ptr<T>((type & 0xff) == BC_DIRICHLET ? M.g.b_dmid : M.g.b_data) + 4 * (size_t)b, qR);
-        inviscid_flux(P.flux, qL, qR, nx, ny, F, sMax);
+        face_inviscid(M, P.flux, qL, qR, nx, ny, F, sMax);
         if (P.viscous) {
             T g1[4][2], g2[4][2], dq[4][2], qa[4], Fv[4];
             load_grad<T>(A.grad, owner, g1);
@@ -1207,19 +1278,19 @@ __device__ void boundary_flux(const DMesh &M, const DPhys &P, const DArrays &A, 
                 dq[k][0] = half(g1[k][0] + g2[k][0]);
                 dq[k][1] = half(g1[k][1] + g2[k][1]);
             }
-            diffusive_flux(pr, mu, qa, dq, nx, ny, Fv);
+            face_viscous(M, pr, mu, qa, dq, nx, ny, Fv);
             for (int k = 0; k < 4; k++) F[k] = F[k] - Fv[k];
         }
         break;
     }
     case BC_INVWALL: {
-        T inv = 1 / qL[0];
+        T inv = ratio(T(1), qL[0]);
         T vp0 = inv * qL[1], vp1 = inv * qL[2];
         T vn = vp0 * nx + vp1 * ny;
         T t0 = vp0 - vn * nx, t1 = vp1 - vn * ny;
-        T vel = dsqrt(t0 * t0 + t1 * t1);
+        T vel = root(t0 * t0 + t1 * t1);
         T p = (G - 1) * (qL[3] - T(0.5) * qL[0] * (vel * vel));
-        T a = dsqrt(G * (p / qL[0]));
+        T a = root(G * ratio(p, qL[0]));
         if (p < 0) p = T(1.0e-12);
         F[0] = 0;
         F[1] = p * nx;
@@ -1231,7 +1302,7 @@ __device__ void boundary_flux(const DMesh &M, const DPhys &P, const DArrays &A, 
     case BC_VISCWALL: {
         T vel = 0.0;
         T p = (G - 1) * (qL[3] - T(0.5) * qL[0] * (vel * vel));
-        T a = dsqrt(G * (p / qL[0]));
+        T a = root(G * ratio(p, qL[0]));
         if (p < 0) p = T(1.0e-12);
         T qR[4] = {qL[0], qL[1] * -1, qL[2] * -1, qL[3]};
         T qa[4], dq[4][2], Fv[4];
@@ -1239,9 +1310,10 @@ __device__ void boundary_flux(const DMesh &M, const DPhys &P, const DArrays &A, 
         qa[1] = 0.0;
         qa[2] = 0.0;
         load_grad<T>(A.grad, owner, dq);
-        dq[3][0] = (qa[3] / qa[0]) * dq[0][0];
-        dq[3][1] = (qa[3] / qa[0]) * dq[0][1];
-        diffusive_flux(pr, mu, qa, dq, nx, ny, Fv);
+        const T e = ratio(qa[3], qa[0]);
+        dq[3][0] = e * dq[0][0];
+        dq[3][1] = e * dq[0][1];
+        face_viscous(M, pr, mu, qa, dq, nx, ny, Fv);
         F[0] = 0 - Fv[0];
         F[1] = p * nx - Fv[1];
         F[2] = p * ny - Fv[2];
@@ -1253,17 +1325,17 @@ __device__ void boundary_flux(const DMesh &M, const DPhys &P, const DArrays &A, 
         T qg[4];
         ld4(qin + 4 * (size_t)ghost, qg);
         T p = pressure(qg);
-        T u = qg[1] / qg[0], v = qg[2] / qg[0];
-        T a = dsqrt(G * (p / qg[0]));
+        T u = ratio(qg[1], qg[0]), v = ratio(qg[2], qg[0]);
+        T a = root(G * ratio(p, qg[0]));
         convective_flux(p, u, v, qg[0], qg[3], nx, ny, F);
         sMax = fabs(a);
         break;
     }
     case BC_SYMMETRY: {
-        T v0 = qL[1] / qL[0], v1 = qL[2] / qL[0], n0, n1;
+        T v0 = ratio(qL[1], qL[0]), v1 = ratio(qL[2], qL[0]), n0, n1;
         reflect(type, ptr<T>(M.g.b_refl) + 4 * (size_t)b, v0, v1, n0, n1);
         T qR[4] = {qL[0], qL[0] * n0, qL[0] * n1, qL[3]};
-        inviscid_flux(P.flux, qL, qR, nx, ny, F, sMax);
+        face_inviscid(M, P.flux, qL, qR, nx, ny, F, sMax);
         if (P.viscous) {
             T gp[4][2], qa[4], Fv[4];
             load_grad<T>(A.grad, owner, gp);
@@ -1288,7 +1360,7 @@ __device__ void boundary_flux(const DMesh &M, const DPhys &P, const DArrays &A, 
                     for (int k = 0; k < 2; k++) a1 += gp[r][k] * nO[k][c];
                     bG[r][c] = a1 + a3;
                 }
-            diffusive_flux(pr, mu, qa, bG, nx, ny, Fv);
+            face_viscous(M, pr, mu, qa, bG, nx, ny, Fv);
             for (int k = 0; k < 4; k++) F[k] = F[k] - Fv[k];
         }
         break;
@@ -1296,12 +1368,12 @@ __device__ void boundary_flux(const DMesh &M, const DPhys &P, const DArrays &A, 
     case BC_TPINFLOW: {
         T qR[4];
         ld4(qin + 4 * (size_t)ghost, qR);
-        inviscid_flux(P.flux, qL, qR, nx, ny, F, sMax);
+        face_inviscid(M, P.flux, qL, qR, nx, ny, F, sMax);
         if (P.viscous) {
             T gp[4][2], qa[4], Fv[4];
             load_grad<T>(A.grad, owner, gp);
             for (int k = 0; k < 4; k++) qa[k] = half(qL[k] + qR[k]);
-            diffusive_flux(pr, mu, qa, gp, nx, ny, Fv);
+            face_viscous(M, pr, mu, qa, gp, nx, ny, Fv);
             for (int k = 0; k < 4; k++) F[k] = F[k] - Fv[k];
         }
         break;
@@ -1423,16 +1495,18 @@ __device__ __forceinline__ bool edge_flux_soft(const DMesh &M, const DPhys &P, c
 template <typename T, int PR>
 __global__ void __launch_bounds__(flux_threads<T, PR>(), flux_minb<T, PR>())
     k_flux(const __grid_constant__ DMesh M, const __grid_constant__ DPhys P, const __grid_constant__ DArrays A,
-           const T *__restrict__ qin, int nbi)
+           const T *__restrict__ qin, int nbb)
 {
-    if ((int)blockIdx.x >= nbi) {
+    // the boundary blocks first: theirs is the longest latency
+    if ((int)blockIdx.x < nbb) {
         grid_dep_release();
         grid_dep_wait();
-        const int b = (blockIdx.x - nbi) * blockDim.x + threadIdx.x;
+        const int b = blockIdx.x * blockDim.x + threadIdx.x;
         if (b < M.G) boundary_flux<T>(M, P, A, qin, b);
         return;
     }
-    const int e = ordered_block(M, nbi) * blockDim.x + threadIdx.x;
+    const int nbi = gridDim.x - nbb, blk = (int)blockIdx.x - nbb;
+    const int e = (M.rev ? nbi - 1 - blk : blk) * blockDim.x + threadIdx.x;
     const bool act = e < M.Eint;
     // read-only mesh data before the wait for the previous kernel
     int inst = 0;
@@ -1521,12 +1595,6 @@ template <> __device__ __forceinline__ void mul4<double>(const double a[4], doub
 #pragma unroll
         for (int k = 0; k < 4; k++) o[k] = ebbsoft::mul(a[k], b);
     }
-}
-// a / b, FP64 on the integer pipe
-template <typename T> __device__ __forceinline__ T ratio(T a, T b) { return a / b; }
-template <> __device__ __forceinline__ double ratio<double>(double a, double b)
-{
-    return ebbdiv::div(a, ebbdiv::recip(b));
 }
 // acc + 2 x (2 x is exact: one rounding)
 template <typename T> __device__ __forceinline__ T plus_twice(T acc, T x) { return acc + T(2.0) * x; }
@@ -2022,7 +2090,7 @@ int launch_flux_pr(const DMesh &M, const DPhys &P, const DArrays &A, const T *qi
     const int TB = flux_threads<T, PR>();
     int nbi = (M.Eint + TB - 1) / TB, nbb = (M.G + TB - 1) / TB;
     if (nbi + nbb == 0) return 0;
-    return ret(launch_dep(k_flux<T, PR>, dim3(nbi + nbb), dim3(TB), (cudaStream_t)stream, M, P, A, qin, nbi));
+    return ret(launch_dep(k_flux<T, PR>, dim3(nbi + nbb), dim3(TB), (cudaStream_t)stream, M, P, A, qin, nbb));
 }
 
 template <typename T, int PR>

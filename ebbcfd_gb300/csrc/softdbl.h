@@ -155,8 +155,11 @@ template <int R> EBB_SOFT_HD void check(double x, bool &bad)
 
 constexpr uint32_t kTop = 0xfff00000u;  // sign and exponent
 
-// RN(a b) for a and b zero or normal whose product is zero or normal
-EBB_SOFT_HD double mul(double a, double b)
+// a 2 for a normal a
+EBB_SOFT_HD double twice(double a) { return make(hi_of(a) + 0x100000u, lo_of(a)); }
+
+// RN(a b) for a and b zero or normal whose product is zero or normal; NZ: a is not zero
+template <bool NZ = false> EBB_SOFT_HD double mul(double a, double b)
 {
     const uint32_t ah = hi_of(a), al = lo_of(a), bh = hi_of(b), bl = lo_of(b);
     const uint32_t Ah = (ah & 0xfffffu) | 0x100000u, Bh = (bh & 0xfffffu) | 0x100000u;
@@ -184,7 +187,7 @@ EBB_SOFT_HD double mul(double a, double b)
     lo = (uint32_t)v;
     hi = (uint32_t)(v >> 32);
 #endif
-    const bool zero = (ah & kExp) == 0u || (bh & kExp) == 0u;
+    const bool zero = (!NZ && (ah & kExp) == 0u) || (bh & kExp) == 0u;
     return make(zero ? (ah ^ bh) & 0x80000000u : hi, zero ? 0u : lo);
 }
 
