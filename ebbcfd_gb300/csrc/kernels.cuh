@@ -1024,7 +1024,7 @@ __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
                 const long long bits = __double_as_longlong(du);
                 dlo = (unsigned long long)bits > (unsigned long long)dlo ? bits : dlo;
                 dhi = bits > dhi ? bits : dhi;
-                const double px = sm<SG_GRAD>(gm.x, du), py = sm<SG_GRAD>(gm.y, du);
+                const double px = sm<SG_GRAD, true>(gm.x, du), py = sm<SG_GRAD, true>(gm.y, du);
                 g0 = j == 0 ? zero_plus(px) : g0 + px;
                 g1 = j == 0 ? zero_plus(py) : g1 + py;
             } else {
@@ -1058,7 +1058,7 @@ __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
                 lim = limit_exact(M, i, UNI ? MJ : ne, qin, k, qi, g0, g1);
             } else if (j >= 0) {
                 const double2 nd = ld2<double>(M.g.s_nd, (size_t)j * Cs + i);
-                const double dd = sm<SG_LIM>(g0, nd.x) + sm<SG_LIM>(g1, nd.y);
+                const double dd = sm<SG_LIM, true>(g0, nd.x) + sm<SG_LIM, true>(g1, nd.y);
                 const double s = soft_ratio(low ? dl : dh, dd, bad);
                 lim = __double2hiint(s) < 0x3ff00000 ? s : 1.0;  // min(1, s), s >= -0
             }
@@ -1085,8 +1085,8 @@ __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
     }
     T lg0, lg1;
     if constexpr (is_fp64<T>) {
-        lg0 = sm<SG_LIM>(lim, g0);
-        lg1 = sm<SG_LIM>(lim, g1);
+        lg0 = sm<SG_LIM, true>(lim, g0);
+        lg1 = sm<SG_LIM, true>(lim, g1);
         ebbsoft::check<400>(lg0, bad);
         ebbsoft::check<400>(lg1, bad);
         if (__any_sync(quad, bad)) {
@@ -1116,7 +1116,7 @@ __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
             const typename V2<T>::t fd = slot(fdk, j);
             T f;
             if constexpr (is_fp64<T>)
-                f = qi + sm<SG_FACE>(lg0, fd.x) + sm<SG_FACE>(lg1, fd.y);
+                f = qi + sm<SG_FACE, true>(lg0, fd.x) + sm<SG_FACE, true>(lg1, fd.y);
             else
                 f = qi + lg0 * fd.x + lg1 * fd.y;
             if (pressure_negative4(f, k, quad)) {
@@ -1189,8 +1189,11 @@ template <typename T> __device__ __forceinline__ bool has_nan(const T F[4])
 }
 
 // The inviscid and viscous flux of a boundary face.  FP64: flux_soft.cuh's where the values
-// allow it.  A boundary block's latency is one face's: with device_math.cuh's ~450 FP64
-// instructions it was all of k_flux on small meshes (13.4 us on 1024 quads).
+// allow it, with its quotients and roots on the integer pipe and its products on the FP64
+// pipe (a third of the code).  A boundary block's latency is one face's, instruction
+// fetches included: with device_math.cuh's ~450 FP64 instructions it was all of k_flux on
+// small meshes (a step of 1024 quads 69 us; 67 us with every product on the integer pipe;
+// so, 62 us).
 template <typename T>
 __device__ __noinline__ void inviscid_plain(int kind, const T qL[4], const T qR[4], T nx, T ny, T F[4], T &sMax)
 {
@@ -1208,7 +1211,7 @@ __device__ __forceinline__ void face_inviscid(const DMesh &M, int kind, const T 
     if constexpr (is_fp64<T>) {
         bool bad = !M.soft;
         double X[4], s;
-        inviscid_flux2_soft(kind, qL, qR, nx, ny, X, s, bad);
+        inviscid_flux2_soft<false>(kind, qL, qR, nx, ny, X, s, bad);
         if (bad) {
             const double a[4] = {qL[0], qL[1], qL[2], qL[3]}, b[4] = {qR[0], qR[1], qR[2], qR[3]};
             inviscid_plain<T>(kind, a, b, nx, ny, X, s);
@@ -1231,7 +1234,7 @@ __device__ __forceinline__ void face_viscous(const DMesh &M, const ViscConst<T> 
 #pragma unroll
         for (int k = 1; k < 4; k++) ebbsoft::check<100>(q[k], bad);
         double X[4];
-        diffusive_flux2_soft(vc, mu, q, dq, nx, ny, X, bad);
+        diffusive_flux2_soft<false>(vc, mu, q, dq, nx, ny, X, bad);
         if (bad) {
             const double a[4] = {q[0], q[1], q[2], q[3]};
             const double g[4][2] = {{dq[0][0], dq[0][1]}, {dq[1][0], dq[1][1]}, {dq[2][0], dq[2][1]}, {dq[3][0], dq[3][1]}};
@@ -1246,7 +1249,7 @@ __device__ __forceinline__ void face_viscous(const DMesh &M, const ViscConst<T> 
 }
 
 template <typename T>
-__device__ void boundary_flux(const DMesh &M, const DPhys &P, const DArrays &A, const T *qin, int b)
+__device__ __forceinline__ void boundary_flux(const DMesh &M, const DPhys &P, const DArrays &A, const T *qin, int b)
 {
     const T G = K<T>::g;
     const int type = M.b_type[b];
@@ -1389,6 +1392,15 @@ __device__ void boundary_flux(const DMesh &M, const DPhys &P, const DArrays &A, 
     if (M.speeds) reinterpret_cast<T *>(A.fs)[e] = len * sMax;
 }
 
+// FP64 and double-float: a call, so that the interior faces' registers and code are theirs
+// alone (500,000 plate cells, double-float: step 827 -> 786 us; split precision is 1 to 5%
+// faster with it in line)
+template <typename T>
+__device__ __noinline__ void boundary_flux_call(const DMesh &M, const DPhys &P, const DArrays &A, const T *qin, int b)
+{
+    boundary_flux<T>(M, P, A, qin, b);
+}
+
 // len * flux and len * sMax of interior edge e from its two face states (and, viscous,
 // its cells' gradients)
 template <typename T>
@@ -1467,7 +1479,7 @@ __device__ __forceinline__ bool edge_flux_soft(const DMesh &M, const DPhys &P, c
 {
     double F[4], sMax;  // F: twice the flux
     bool bad = false;
-    inviscid_flux2_soft(P.flux, qL, qR, n.x, n.y, F, sMax, bad);
+    inviscid_flux2_soft<true>(P.flux, qL, qR, n.x, n.y, F, sMax, bad);
     if (P.viscous) {
         const int2 c = make_int2(slot_cell(M, sl.x), slot_cell(M, sl.y));
         double g1[4][2], g2[4][2], Fv[4];
@@ -1479,7 +1491,7 @@ __device__ __forceinline__ bool edge_flux_soft(const DMesh &M, const DPhys &P, c
             g1[k][0] = g1[k][0] + g2[k][0];
             g1[k][1] = g1[k][1] + g2[k][1];
         }
-        diffusive_flux2_soft(visc_const<double>(P), visc_mu<double>(M, P, inst), qL, g1, n.x, n.y, Fv, bad);
+        diffusive_flux2_soft<true>(visc_const<double>(P), visc_mu<double>(M, P, inst), qL, g1, n.x, n.y, Fv, bad);
         F[0] = F[0] - zero_dot(n.x, n.y);
 #pragma unroll
         for (int k = 1; k < 4; k++) F[k] = F[k] - Fv[k];
@@ -1502,7 +1514,12 @@ __global__ void __launch_bounds__(flux_threads<T, PR>(), flux_minb<T, PR>())
         grid_dep_release();
         grid_dep_wait();
         const int b = blockIdx.x * blockDim.x + threadIdx.x;
-        if (b < M.G) boundary_flux<T>(M, P, A, qin, b);
+        if (b < M.G) {
+            if constexpr (is_fp32<T>)
+                boundary_flux<T>(M, P, A, qin, b);
+            else
+                boundary_flux_call<T>(M, P, A, qin, b);
+        }
         return;
     }
     const int nbi = gridDim.x - nbb, blk = (int)blockIdx.x - nbb;
