@@ -1613,6 +1613,14 @@ template <> __device__ __forceinline__ void mul4<double>(const double a[4], doub
         for (int k = 0; k < 4; k++) o[k] = ebbsoft::mul(a[k], b);
     }
 }
+// x with its sign changed where bit 31 of s is set.  (Two branches, one with -x, ran both
+// in nearly every warp: edges of either orientation alternate from cell to cell.)
+__device__ __forceinline__ float flip(float x, int s) { return __int_as_float(__float_as_int(x) ^ (s & 0x80000000)); }
+__device__ __forceinline__ double flip(double x, int s)
+{
+    return __hiloint2double(__double2hiint(x) ^ (s & 0x80000000), __double2loint(x));
+}
+__device__ __forceinline__ df flip(df x, int s) { return df(flip(x.hi, s), flip(x.lo, s)); }
 // acc + 2 x (2 x is exact: one rounding)
 template <typename T> __device__ __forceinline__ T plus_twice(T acc, T x) { return acc + T(2.0) * x; }
 template <> __device__ __forceinline__ double plus_twice<double>(double acc, double x) { return fma(2.0, x, acc); }
@@ -1715,17 +1723,12 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
             if (j < ne) {
                 if (is_fp64<T> && j == 0) {  // 0 + x without the FP64 pipe
 #pragma unroll
-                    for (int k = 0; k < 4; k++) r[k] = zero_plus(ev[0] < 0 ? -f[0][k] : f[0][k]);
+                    for (int k = 0; k < 4; k++) r[k] = zero_plus(flip(f[0][k], ev[0]));
                     sAve = fe[0];
                     continue;
                 }
-                if (ev[j] < 0) {
 #pragma unroll
-                    for (int k = 0; k < 4; k++) r[k] = r[k] + (-f[j][k]);
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 4; k++) r[k] = r[k] + f[j][k];
-                }
+                for (int k = 0; k < 4; k++) r[k] = r[k] + flip(f[j][k], ev[j]);
                 sAve += fe[j];
             }
         }
@@ -1753,17 +1756,12 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
 #pragma unroll
             for (int j = 0; j < MJ; j++) {
                 if (j < ne) {
-                    const T len = sl[j];
+                    const T len = flip(sl[j], ev[j]);
                     T F[4];
                     convective_flux(pc, uc, vc, qc[0], qc[3], sn[j].x, sn[j].y, F);
                     // len F rounded on its own, as k_flux stores it (no contraction)
-                    if (ev[j] < 0) {
 #pragma unroll
-                        for (int k = 0; k < 4; k++) c[k] = __fadd_rn(c[k], -__fmul_rn(len, F[k]));
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < 4; k++) c[k] = __fadd_rn(c[k], __fmul_rn(len, F[k]));
-                    }
+                    for (int k = 0; k < 4; k++) c[k] = __fadd_rn(c[k], __fmul_rn(len, F[k]));
                 }
             }
 #pragma unroll
@@ -2001,52 +1999,58 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
         }
         return;
     } else if constexpr (!SPLIT) {
-        // FP64: every thread's values go to shared memory, and whole warps reduce
-        // columns, one lane per (column, group of 16 rows): an FP64 warp instruction
-        // costs the same with 1 or 32 lanes active, so a shuffle tree per value (5
-        // levels x 10 values per warp) would spend most of the kernel's FP64 time here.
-        // Column 1 holds -Rmax so that every column of warp 0 is a min.  Fixed order.
-        constexpr int W = 11;  // row stride in doubles: conflict-free strided reads
-        __shared__ double shr[UPD_THREADS * W];
-        __shared__ double part[10][16];
-        const int t = threadIdx.x;
-        const int ncol = final_stage ? 10 : 2;
-        shr[t * W + 0] = dtc;
-        shr[t * W + 1] = -rm;
+        // The smallest time step and the largest residual as integers (non-negative doubles
+        // order as their bit patterns).  The eight sums, FP64, by halving: at each of the
+        // first three exchanges a lane keeps half of its columns, so a warp adds 9 times
+        // where a shuffle tree per column adds 40 (an FP64 instruction costs a warp 64
+        // cycles with 1 lane active as with 32).  Fixed order.
+        constexpr int NW = UPD_THREADS / 32;
+        constexpr unsigned all = 0xffffffffu;
+        __shared__ unsigned long long key[NW][2];
+        __shared__ double shr[NW][8];
+        if (need_dt) {
+            const unsigned long long d = (unsigned long long)__double_as_longlong(dtc != dtc ? INFINITY : dtc);
+            const unsigned h = __reduce_min_sync(all, (unsigned)(d >> 32));
+            const unsigned l = __reduce_min_sync(all, (unsigned)(d >> 32) == h ? (unsigned)d : all);
+            if (lane == 0) key[w][0] = ((unsigned long long)h << 32) | l;
+        }
+        const unsigned long long m = (unsigned long long)__double_as_longlong(rm);
+        const unsigned h = __reduce_max_sync(all, (unsigned)(m >> 32));
+        const unsigned l = __reduce_max_sync(all, (unsigned)(m >> 32) == h ? (unsigned)m : 0u);
+        if (lane == 0) key[w][1] = ((unsigned long long)h << 32) | l;
         if (final_stage) {
+            double v[8] = {ss[0], ss[1], ss[2], ss[3], vs[0], vs[1], vs[2], vs[3]};
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                shr[t * W + 2 + k] = ss[k];
-                shr[t * W + 6 + k] = vs[k];
+            for (int n = 4, o = 16; n > 0; n >>= 1, o >>= 1) {
+                const bool up = lane & o;
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (k < n) {
+                        const double keep = up ? v[n + k] : v[k], give = up ? v[k] : v[n + k];
+                        v[k] = keep + __shfl_xor_sync(all, give, o);
+                    }
             }
+            v[0] = v[0] + __shfl_xor_sync(all, v[0], 2);
+            v[0] = v[0] + __shfl_xor_sync(all, v[0], 1);
+            if ((lane & 3) == 0) shr[w][lane >> 2] = v[0];  // column: the kept halves' bits
         }
         __syncthreads();
-        if (t < 16 * ncol) {  // group g of column c: rows g, g+16, ..., g+240
-            const int c = t >> 4, g = t & 15;
-            double a = shr[g * W + c];
-            if (c < 2) {
-                for (int r = 1; r < UPD_THREADS / 16; r++) a = fmin(a, shr[(g + 16 * r) * W + c]);
-            } else {
-                for (int r = 1; r < UPD_THREADS / 16; r++) a = a + shr[(g + 16 * r) * W + c];
-            }
-            part[c][g] = a;
+        if (w != 0) return;
+        if (final_stage) {
+            const int c = lane & 7, g = lane >> 3;
+            double v = shr[g][c];
+            for (int k = g + 4; k < NW; k += 4) v = v + shr[k][c];
+            v = v + __shfl_xor_sync(all, v, 8);
+            v = v + __shfl_xor_sync(all, v, 16);
+            if (lane < 8) A.red[8 * (size_t)blk + c] = v;
         }
-        __syncthreads();
-        if (t < ncol) {
-            double a = part[t][0];
-            if (t < 2) {
-                for (int g = 1; g < 16; g++) a = fmin(a, part[t][g]);
-            } else {
-                for (int g = 1; g < 16; g++) a = a + part[t][g];
-            }
-            if (t == 0) {
-                if (need_dt && a == a) atomicMin(&st->newdt_bits, (unsigned long long)__double_as_longlong(a));
-            } else if (t == 1) {
-                const double b = -a;
-                if (b > 0) atomicMax(&st->rmax_bits, (unsigned long long)__double_as_longlong(b));
-            } else {
-                A.red[8 * (size_t)blk + (t - 2)] = a;
-            }
+        if (lane < 2 && (lane == 1 || need_dt)) {
+            unsigned long long x = key[0][lane];
+            for (int k = 1; k < NW; k++) x = lane ? max(x, key[k][1]) : min(x, key[k][0]);
+            if (lane == 0)
+                atomicMin(&st->newdt_bits, x);
+            else if (x != 0ull)
+                atomicMax(&st->rmax_bits, x);
         }
     }
 }

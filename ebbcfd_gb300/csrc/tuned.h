@@ -6,14 +6,15 @@
 // split k_flux: 64x16 133.7 us, 64x20 124.0 us, 128x8 135.0 us, 128x10 124.9 us, 128x12 115.8 us, 256x4 149.2 us, 256x6 119.7 us
 // split k_update: 256x4 135.6 us, 256x6 137.6 us, 256x8 150.3 us, 512x2 140.3 us, 512x3 143.8 us, 512x4 156.8 us
 // fp64 (400,000 cells, by hand) k_cell: 128x4 151.8 us, 128x6 142.9 us; k_flux: 128x4 194.7 us, 128x5 200.9 us,
-// 128x6 202.2 us; k_update: 256x4 49.8 us
+// 128x6 202.2 us; k_update: 256x3 32.6 us, 256x4 32.4 us
 // df k_cell: 64x4 1035.3 us, 64x6 1026.0 us, 128x1 1018.2 us, 128x2 1018.4 us, 128x3 1017.0 us, 256x1 1355.9 us, 256x2 824.7 us
 // df (500,000 cells, by hand) k_flux: 128x5 61.5 us, 128x6 62.2 us, 128x8 63.3 us
 // df k_update: 256x1 409.5 us, 256x2 409.6 us, 256x3 293.6 us, 256x4 256.0 us, 512x1 465.2 us, 512x2 289.0 us
 // split_inv k_cell: 64x12 30.9 us, 64x16 27.4 us, 128x6 31.9 us, 128x8 27.8 us, 128x10 32.5 us, 256x3 32.8 us, 256x4 27.8 us
 // split_inv k_flux: 64x16 27.0 us, 64x20 26.9 us, 128x8 23.4 us, 128x10 22.3 us, 128x12 20.3 us, 256x4 25.4 us, 256x6 20.9 us
 // split_inv k_update: 256x4 32.3 us, 256x6 30.0 us, 256x8 28.9 us, 512x2 35.3 us, 512x3 30.6 us, 512x4 29.3 us
-// split_inv k_update since (500,000 cells, by hand): 256x4 11.6 us, 256x5 11.5 us, 256x6 14.0 us, 256x7 15.1 us
+// split k_update since (1M cells, by hand): 256x3 34.1 us, 256x4 35.4 us; df (500,000): 256x3 28.0 us, 256x4 28.9 us
+// split_inv k_update since (500,000 cells, by hand): 256x5 11.2 us, 256x6 13.5 us
 // update block size 256 (summed best update times: 256: 987.6 us, 512: 1063.9 us)
 #pragma once
 #ifndef EBB_CELL_TB_F
@@ -56,13 +57,13 @@
 #define EBB_UPD_TB 256
 #endif
 #ifndef EBB_UPD_MINB_F
-#define EBB_UPD_MINB_F 4
+#define EBB_UPD_MINB_F 3
 #endif
 #ifndef EBB_UPD_MINB_D
-#define EBB_UPD_MINB_D 4
+#define EBB_UPD_MINB_D 3
 #endif
 #ifndef EBB_UPD_MINB_W
-#define EBB_UPD_MINB_W 4
+#define EBB_UPD_MINB_W 3
 #endif
 #ifndef EBB_CELL_TB_FI
 #define EBB_CELL_TB_FI 64
