@@ -831,25 +831,24 @@ __device__ __noinline__ void cell_plain(const DMesh &M, const DPhys &P, const DA
 }
 
 // The scalar limiter of one component (solve.d:336-402) on the integer and FP32 pipes.
-// dl <= 0 <= dh are the bounds minus the cell's value.  Which neighbours' extrapolations
+// lo <= 0 <= hi are FP32 values of the bounds minus the cell's value (lo0, hi0: exactly
+// zero), g0f and g1f of the gradient (flat: exactly zero).  Which neighbours' extrapolations
 // leave the bounds, and which of those gives the smallest ratio, is decided in FP32 from
-// values truncated to 23 bits; a decision that is not clear of the truncation and rounding
-// errors sets `unsure` (limit_exact then decides; measured on smooth flows: 2 to 3 of
-// 1,000 cells).  Returns the deciding neighbour, or -1; `low` tells its bound.
+// values good to 23 bits; a decision that is not clear of their errors and of M, the
+// rounding of the cell's value plus a difference, sets `unsure` (limit_exact then decides;
+// measured on smooth flows: 2 to 3 of 1,000 cells).  Returns the deciding neighbour, or -1;
+// `low` tells its bound.
 //
-// With dd = RN(RN(g0 nx) + RN(g1 ny)) and e its FP32 value: |e - dd| < 2^-21 (|a| + |b|),
-// the FP32 bounds are within 2^-23 of theirs, and RN(q + dd) compares with a bound as dd
-// does with its difference when they are 2^-51 |q| apart.
+// With dd = g0 nx + g1 ny in the form's arithmetic and e its FP32 value: |e - dd| < 2^-21
+// (|a| + |b|), the FP32 bounds are within 2^-23 of theirs, and q + dd compares with a bound
+// as dd does with its difference when they are M / 2 apart (FP64: 2^-51 |q|).
 template <int MJ>
-__device__ __forceinline__ int limiting_neighbour(double q, double g0, double g1, double dl, double dh,
-                                                  const float (&nx)[MJ], const float (&ny)[MJ], int ne, bool &low,
-                                                  bool &unsure)
+__device__ __forceinline__ int limiting_neighbour(float M, float g0f, float g1f, bool flat, float lo, float hi, bool lo0,
+                                                  bool hi0, const float (&nx)[MJ], const float (&ny)[MJ], int ne,
+                                                  bool &low, bool &unsure)
 {
-    const float g0f = trunc_sat(g0), g1f = trunc_sat(g1), lo = trunc_sat(dl), hi = trunc_sat(dh);
-    const float M = __fadd_rn(0x1p-50f * fabsf(trunc_sat(q)), 0x1p-100f);
     const float ml = __fmaf_rn(0x1p-21f, fabsf(lo), M), mh = __fmaf_rn(0x1p-21f, hi, M);
     const float lo_out = lo - ml, lo_in = lo + ml, hi_out = hi + mh, hi_in = hi - mh;
-    const bool flat = g0 == 0.0 && g1 == 0.0;  // every extrapolation is the cell's value
     int best = -1;
     float s1 = 4.0f, up1 = 4.0f, dn1 = 4.0f, dn2 = 8.0f;  // the smallest ratio and its interval, the others' lower end
 #pragma unroll
@@ -877,7 +876,7 @@ __device__ __forceinline__ int limiting_neighbour(double q, double g0, double g1
         }
     }
     // two ratios too close to tell apart (a zero one is the smallest: its bound is exact)
-    if (best >= 0) unsure |= (low ? dl : dh) != 0.0 && !(s1 > 0x1p-60f && dn2 > up1);
+    if (best >= 0) unsure |= !(low ? lo0 : hi0) && !(s1 > 0x1p-60f && dn2 > up1);
     return best;
 }
 
@@ -898,6 +897,18 @@ __device__ __forceinline__ double limit_exact(const DMesh &M, int i, int ne, con
         const double2 nd = ld2<double>(M.g.s_nd, (size_t)j * M.Cs + i);
         const double dd = g0 * nd.x + g1 * nd.y, qE = q + dd;
         if (qE < mn || qE > mx) l = fmin(l, ebbdiv::div((qE < mn ? mn : mx) - q, ebbdiv::recip(dd)));
+    }
+    return l;
+}
+
+__device__ __forceinline__ df limit_exact(const DMesh &M, int i, int ne, df g0, df g1, df dl, df dh)
+{
+    df l = df(1.0f);
+#pragma unroll 1
+    for (int j = 0; j < ne; j++) {
+        const df2 nd = ld2<df>(M.g.s_nd, (size_t)j * M.Cs + i);
+        const df dd = g0 * nd.x + g1 * nd.y;
+        if (dd < dl || dd > dh) l = fmin(l, (dd < dl ? dl : dh) / dd);
     }
     return l;
 }
@@ -938,20 +949,21 @@ __device__ __forceinline__ bool pressure_negative4(df x, int, unsigned quad)
 // quarter of the values: the registers of one thread per cell (80 and 128 of them) kept
 // 24 and 16 warps on an SM, too few to cover the latency of either form's arithmetic.
 //
-// FP64: the products, the limiter's decisions and its quotients run on the integer and
-// FP32 pipes (softdbl.h) beside the FP64 pipe; the values are cell_body's bit for bit,
-// and a cell with a value out of that arithmetic's range goes to cell_plain.  Bound by
-// the FP64 pipe's additions (61% busy; integer pipe 50%, a sixth of the time fetching
-// instructions).  Double-float: issue (66% of the slots).
+// The limiter's decisions are taken in FP32 (limiting_neighbour), so that one quotient per
+// component is formed.  FP64: the products and that quotient run on the integer pipe
+// (softdbl.h) beside the FP64 pipe; the values are cell_body's bit for bit, and a cell with
+// a value out of that arithmetic's range goes to cell_plain.  Bound by the FP64 pipe's
+// additions (61% busy; integer pipe 50%, a sixth of the time fetching instructions).
+// Double-float: x and y in packed operations (dfpair.cuh), bound by issue.
 //
 // Lane k loads the geometry of slot k before the wait for the previous kernel: with each
 // lane loading every slot's where it is used, loads from memory took 45% (FP64) and 63%
 // (double-float) of the warps' time.
 //
 // Measured against one thread per cell, us per launch, FP64 / double-float: 400,000 plate
-// cells 140 (143) / 84 (109); 200,000 triangles 53 (52) / 28 (36); 1024 quads, where one
-// warp's latency is the launch's, 7.5 (16.3) / 5.6 (14.1).  FP64 steps: 1,815 (1,879),
-// 318 (329) and 76 (91) us.
+// cells 145 (318 all on the FP64 pipe, 143 as here) / 76 (109); 200,000 triangles 54 (155,
+// 52) / 25 (36); 1024 quads, where one warp's latency is the launch's, 7.3 (23, 16) / 5.3
+// (14).
 template <typename T, int MJ, bool UNI>
 __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
     k_cell4(const __grid_constant__ DMesh M, const __grid_constant__ DPhys P, const __grid_constant__ DArrays A,
@@ -1003,8 +1015,9 @@ __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
         return o;
     };
     bool bad = false;
-    T g0 = T(0.0), g1 = T(0.0), mn = qi, mx = qi;
-    long long dlo = 0, dhi = 0;  // FP64: bit patterns of the smallest and largest neighbour difference
+    T g0 = T(0.0), g1 = T(0.0), dl = T(0.0), dh = T(0.0);  // smallest and largest neighbour difference, or 0
+    long long dlo = 0, dhi = 0;                            // FP64: their bit patterns
+    dfp gp = pair(df(0.0f), df(0.0f));                     // double-float: the gradient
 #pragma unroll
     for (int j = 0; j < MJ; j++) {
         if (UNI || j < ne) {
@@ -1028,59 +1041,67 @@ __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
                 g0 = j == 0 ? zero_plus(px) : g0 + px;
                 g1 = j == 0 ? zero_plus(py) : g1 + py;
             } else {
-                mn = fmin(mn, qv[j]);
-                mx = fmax(mx, qv[j]);
-                g0 = g0 + gm.x * du;
-                g1 = g1 + gm.y * du;
+                if (du < dl) dl = du;
+                if (du > dh) dh = du;
+                const dfp p = pair(gm.x, gm.y) * both(du);
+                gp = j == 0 ? p : gp + p;
             }
         }
     }
-    T lim = T(1.0);
+    float g0f, g1f, lo, hi, mar;
     if constexpr (is_fp64<T>) {
         ebbsoft::check<200>(g0, bad);
         ebbsoft::check<200>(g1, bad);
-        if (P.limited && limit) {
-            float nx[MJ], ny[MJ], nxk[H], nyk[H];
+        dl = dlo < 0 ? __longlong_as_double(dlo) : 0.0;
+        dh = __longlong_as_double(dhi);
+        g0f = trunc_sat(g0);
+        g1f = trunc_sat(g1);
+        lo = trunc_sat(dl);
+        hi = trunc_sat(dh);
+        mar = __fadd_rn(0x1p-50f * fabsf(trunc_sat(qi)), 0x1p-100f);
+    } else {
+        split(gp, g0, g1);
+        g0f = g0.hi;
+        g1f = g1.hi;
+        lo = dl.hi;
+        hi = dh.hi;
+        mar = __fadd_rn(0x1p-43f * fabsf(qi.hi), 0x1p-100f);
+    }
+    T lim = T(1.0);
+    if (P.limited && limit) {
+        float nx[MJ], ny[MJ], nxk[H], nyk[H];
 #pragma unroll
-            for (int h = 0; h < H; h++) {
+        for (int h = 0; h < H; h++) {
+            if constexpr (is_fp64<T>) {
                 nxk[h] = trunc_sat(ndk[h].x);
                 nyk[h] = trunc_sat(ndk[h].y);
+            } else {
+                nxk[h] = ndk[h].x.hi;
+                nyk[h] = ndk[h].y.hi;
             }
+        }
 #pragma unroll
-            for (int j = 0; j < MJ; j++) {
-                nx[j] = __shfl_sync(quad, nxk[j >> 2], j & 3, 4);
-                ny[j] = __shfl_sync(quad, nyk[j >> 2], j & 3, 4);
-            }
-            const double dl = dlo < 0 ? __longlong_as_double(dlo) : 0.0, dh = __longlong_as_double(dhi);
-            bool low = false, unsure = false;
-            const int j = limiting_neighbour<MJ>(qi, g0, g1, dl, dh, nx, ny, UNI ? MJ : ne, low, unsure);
-            if (unsure) {
+        for (int j = 0; j < MJ; j++) {
+            nx[j] = __shfl_sync(quad, nxk[j >> 2], j & 3, 4);
+            ny[j] = __shfl_sync(quad, nyk[j >> 2], j & 3, 4);
+        }
+        bool low = false, unsure = false;
+        const int j = limiting_neighbour<MJ>(mar, g0f, g1f, g0 == T(0.0) && g1 == T(0.0), lo, hi, dl == T(0.0),
+                                             dh == T(0.0), nx, ny, UNI ? MJ : ne, low, unsure);
+        if (unsure) {
+            if constexpr (is_fp64<T>)
                 lim = limit_exact(M, i, UNI ? MJ : ne, qin, k, qi, g0, g1);
-            } else if (j >= 0) {
-                const double2 nd = ld2<double>(M.g.s_nd, (size_t)j * Cs + i);
+            else
+                lim = limit_exact(M, i, UNI ? MJ : ne, g0, g1, dl, dh);
+        } else if (j >= 0) {
+            const typename V2<T>::t nd = ld2<T>(M.g.s_nd, (size_t)j * Cs + i);
+            if constexpr (is_fp64<T>) {
                 const double dd = sm<SG_LIM, true>(g0, nd.x) + sm<SG_LIM, true>(g1, nd.y);
                 const double s = soft_ratio(low ? dl : dh, dd, bad);
                 lim = __double2hiint(s) < 0x3ff00000 ? s : 1.0;  // min(1, s), s >= -0
+            } else {
+                lim = fmin(lim, (low ? dl : dh) / sum(gp * pair(nd.x, nd.y)));
             }
-        }
-    } else if (P.limited && limit) {
-        // which extrapolations leave the bounds first, then only their quotients
-        unsigned need = 0, above = 0;
-#pragma unroll
-        for (int j = 0; j < MJ; j++) {
-            if (UNI || j < ne) {
-                const typename V2<T>::t nd = slot(ndk, j);
-                const T qE = qi + (g0 * nd.x + g1 * nd.y);
-                const bool lo = qE < mn, hi = qE > mx;
-                if (lo || hi) need |= 1u << j;
-                if (!lo && hi) above |= 1u << j;
-            }
-        }
-        while (need) {
-            const int j = __ffs(need) - 1;
-            need &= need - 1;
-            const typename V2<T>::t nd = ld2<T>(M.g.s_nd, (size_t)j * Cs + i);
-            lim = fmin(lim, ((above >> j & 1u) ? mx - qi : mn - qi) / (g0 * nd.x + g1 * nd.y));
         }
     }
     T lg0, lg1;
@@ -1094,19 +1115,19 @@ __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
             return;
         }
     } else {
-        lg0 = lim * g0;
-        lg1 = lim * g1;
+        gp = both(lim) * gp;
     }
-    typename V2<T>::t pair;
     if (P.need_grad) {
-        pair.x = g0;
-        pair.y = g1;
-        reinterpret_cast<typename V2<T>::t *>(A.grad)[4 * (size_t)i + k] = pair;
+        typename V2<T>::t v;
+        v.x = g0;
+        v.y = g1;
+        reinterpret_cast<typename V2<T>::t *>(A.grad)[4 * (size_t)i + k] = v;
     }
     if (A.lim) {  // limiter values, exported for ebb-reconstruct
-        pair.x = lim;
-        pair.y = lim;
-        reinterpret_cast<typename V2<T>::t *>(A.lim)[4 * (size_t)i + k] = pair;
+        typename V2<T>::t v;
+        v.x = lim;
+        v.y = lim;
+        reinterpret_cast<typename V2<T>::t *>(A.lim)[4 * (size_t)i + k] = v;
     }
     T *face = reinterpret_cast<T *>(A.face);
 #pragma unroll
@@ -1115,10 +1136,13 @@ __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
             const size_t s = (size_t)j * Cs + i;
             const typename V2<T>::t fd = slot(fdk, j);
             T f;
-            if constexpr (is_fp64<T>)
+            if constexpr (is_fp64<T>) {
                 f = qi + sm<SG_FACE, true>(lg0, fd.x) + sm<SG_FACE, true>(lg1, fd.y);
-            else
-                f = qi + lg0 * fd.x + lg1 * fd.y;
+            } else {
+                df x, y;
+                split(gp * pair(fd.x, fd.y), x, y);
+                f = qi + x + y;
+            }
             if (pressure_negative4(f, k, quad)) {
                 T l = fmin(T(1.0), shfl4(quad, lim, 0));
                 l = fmin(l, shfl4(quad, lim, 1));
