@@ -200,12 +200,12 @@ __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.w
 __device__ __forceinline__ void grid_dep_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // This launch's block of index blockIdx.x out of n: the kernels of a stage run through the
-// mesh in opposite directions (DMesh::rev), so each starts with what the one before it has
-// left in the L2 cache.  With the read-once arrays marked to leave it first (`stream`), no
-// stored edge cells, the split update reading normals by edge instead of a copy by slot and
-// wave speeds written and read in the stages that use them only: split steps of 1M plate
-// cells 450 -> 437 us, of 500,000 triangles 91 -> 87 us (k_flux then writes 0.1 MB of its
-// 15 MB to memory), double-float ones of 200,000 triangles 166 -> 149 us.
+// mesh in opposite directions (DMesh::rev; k_cell always forward), so each starts with what
+// the one before it has left in the L2 cache.  With the read-once arrays marked to leave it
+// first (`stream`), no stored edge cells, the split update reading normals by edge instead
+// of a copy by slot and wave speeds written and read in the stages that use them only: split
+// steps of 1M plate cells 450 -> 437 us, of 500,000 triangles 91 -> 87 us (k_flux then writes
+// 0.1 MB of its 15 MB to memory), double-float ones of 200,000 triangles 166 -> 149 us.
 __device__ __forceinline__ int ordered_block(const DMesh &M, int n)
 {
     return M.rev ? n - 1 - (int)blockIdx.x : (int)blockIdx.x;
@@ -576,7 +576,6 @@ __device__ __forceinline__ void cell_body(const DMesh &M, const DPhys &P, const 
         for (int j = 0; j < MJ; j++) pre.nb[j] = (j < ne) ? pre.nb[j] : i;
 #pragma unroll
         for (int j = 0; j < MJ; j++) ld4(qin + 4 * (size_t)(pre.nb[j] < M.C ? pre.nb[j] : i), qv[j]);
-        if (halted(st)) return;  // behind the gathers: they and this test wait together
 #pragma unroll
         for (int j = 0; j < MJ; j++) {
             if (j < ne) {
@@ -1155,12 +1154,20 @@ __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
     }
 }
 
+// One thread per cell: split precision, and the forms k_cell4 does not take.  Bound by the
+// gathers' latency at the registers' limit on warps, so nothing here may cost a register
+// of the split viscous form (80 of 85): its blocks run in ascending order only (a reversible
+// order spills 40 bytes a thread instead of 16), the test for a stopped solve comes before
+// the gathers, and the geometry takes plain loads; inviscid meshes, with registers to
+// spare, mark it to leave L2 first (500,000 triangles 83.8 against 86.3 us a step).  Measured
+// so, per launch and step: 1M plate cells 47.9 -> 39.1 and 424 -> 409 us, 200,000 9.2 -> 8.6
+// and 99.1 -> 98.2 us.
 template <typename T, int MJ, bool LP, bool UNI, int PR>
 __global__ void __launch_bounds__(cell_threads<T, PR>(), cell_minb<T, PR>())
     k_cell(const __grid_constant__ DMesh M, const __grid_constant__ DPhys P, const __grid_constant__ DArrays A,
            const T *__restrict__ qin, int limit)
 {
-    const int i = ordered_block(M, gridDim.x) * blockDim.x + threadIdx.x;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool act = i < M.C;
     // read-only mesh data first, before the wait for the previous kernel.  Split path:
     // the neighbour rows are loaded whatever the cell's edge count (rows past it hold
@@ -1173,13 +1180,17 @@ __global__ void __launch_bounds__(cell_threads<T, PR>(), cell_minb<T, PR>())
         if (M.cell_inst) inst = M.cell_inst[i];
         if constexpr (sizeof(T) == 4) {
             const int Cs = M.Cs;
-#pragma unroll
-            for (int j = 0; j < MJ; j++) pre.nb[j] = stream(M.s_nbr + (size_t)j * Cs + i);
+            const auto geom = [](const void *p, size_t s) { return PR ? lds2<T>(p, s) : ld2<T>(p, s); };
 #pragma unroll
             for (int j = 0; j < MJ; j++) {
-                pre.gm[j] = lds2<T>(M.g.s_gm, (size_t)j * Cs + i);
-                pre.nd[j] = lds2<T>(M.g.s_nd, (size_t)j * Cs + i);
-                pre.fd[j] = lds2<T>(M.g.s_fd, (size_t)j * Cs + i);
+                const int *p = M.s_nbr + (size_t)j * Cs + i;
+                pre.nb[j] = PR ? stream(p) : *p;
+            }
+#pragma unroll
+            for (int j = 0; j < MJ; j++) {
+                pre.gm[j] = geom(M.g.s_gm, (size_t)j * Cs + i);
+                pre.nd[j] = geom(M.g.s_nd, (size_t)j * Cs + i);
+                pre.fd[j] = geom(M.g.s_fd, (size_t)j * Cs + i);
             }
         }
     }
@@ -1187,7 +1198,7 @@ __global__ void __launch_bounds__(cell_threads<T, PR>(), cell_minb<T, PR>())
     grid_dep_wait();
     if (!act) return;
     DState *st = A.st + inst;
-    if (!is_fp32<T> && halted(st)) return;
+    if (halted(st)) return;
     cell_body<T, MJ, LP>(M, P, A, st, i, UNI ? MJ : ne, qin, limit, pre);
 }
 

@@ -6,6 +6,7 @@
 #include <map>
 #include <mutex>
 #include <thread>
+#include <type_traits>
 
 #include "solver_impl.hpp"
 
@@ -119,12 +120,14 @@ inline double bitsd(unsigned long long u)
 }
 
 // One stage's three kernels, each through the mesh in the other direction than the one
-// before it (`odd`: the stage's number in its step is odd).
+// before it (`odd`: the stage's number in its step is odd); split precision, whose cell
+// kernel runs forward only, always forward, backward, forward (1M plate cells 411 -> 409 us).
 template <typename T>
 int run_stage_t(ebb_solver *s, int stage, T *qin, T *qout, int limit, int dt_update, int need_dt, int final_stage,
                 int odd = 0)
 {
     DMesh M = s->M;
+    if (std::is_same<T, float>::value) odd = 0;
     M.speeds = need_dt || (s->P.local_ts && dt_update);
     M.rev = odd;
     CKL(launch_cell<T>(M, s->P, s->A, qin, limit, s->stream));
