@@ -123,12 +123,12 @@ __device__ __forceinline__ dfp recip(dfp b)
     l = fma2(fma2(l, nh, r), r0, l);
     return fast_two_sum2(q, l);
 }
-// sqrt of both, which are positive (a zero, negative or NaN element by dfloat.h's sqrt)
+// sqrt of both, which are positive normal numbers (any other element by dfloat.h's sqrt)
 __device__ __forceinline__ dfp root(dfp a)
 {
     float x, y;
     unpack2(a.hi, x, y);
-    if (!(x > 0.0f && y > 0.0f)) return pair(sqrt(first(a)), sqrt(second(a)));
+    if (!(x >= 0x1p-126f && y >= 0x1p-126f)) return pair(sqrt(first(a)), sqrt(second(a)));
     const f2 r = pack2(ebbdf::rsqrt32(x), ebbdf::rsqrt32(y)), h = mul2(pack2(0.5f, 0.5f), r);
     f2 s = mul2(a.hi, r);
     s = fma2(fma2(neg2(s), s, a.hi), h, s);
