@@ -1,5 +1,6 @@
 """csrc/dfloat.h over FP32's whole range, with first approximations as the device's
-instructions give them: off by up to 2^-22.9, and flushing what is not a normal number."""
+instructions give them: off by up to 2^-22.9, that of the root flushing what is not a normal
+number."""
 import os
 import subprocess
 
@@ -15,7 +16,7 @@ static std::mt19937_64 g(3);
 static double u01() { return (double)(g() >> 11) * 0x1p-53; }
 static float off(double y) { return (float)(y * (1.0 + (2.0 * u01() - 1.0) * 0x1.12p-23)); }
 static float flush(float x) { return std::fabs(x) < 0x1p-126f ? std::copysign(0.0f, x) : x; }
-#define EBB_HOST_RCP(x) flush(off(1.0 / (double)flush(x)))
+#define EBB_HOST_RCP(x) off(1.0 / (double)(x))
 #define EBB_HOST_RSQRT(x) flush(off(1.0 / std::sqrt((double)flush(x))))
 #include "dfloat.h"
 using ebbdf::df;

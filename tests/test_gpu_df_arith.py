@@ -96,3 +96,24 @@ def test_double_float_roots_over_the_range(probe, e0, e1, tol):
         assert (r[~pos] == 0.0).all()
         err = np.abs(value(r)[pos] / exact[pos] - 1)
         assert np.isfinite(err).all() and err.max() <= tol
+
+
+@pytest.mark.parametrize("e0,e1,f0,f1", [(-127, -127, 30, 60), (-126, -100, 26, 60), (-20, 20, -20, 20), (100, 126, -60, 0),
+                                         (127, 127, -60, -1)])
+def test_double_float_quotients_over_the_range(probe, e0, e1, f0, f1):
+    """Divisors of exponents e0..e1 -- from half the smallest normal number to the largest
+    exponent, where a reciprocal or a divisor is subnormal -- and quotients of exponents
+    f0..f1, which keep every remainder an FP32 number: within 2^-44.  Reciprocals in pairs,
+    within that and a unit of the smallest subnormal."""
+    rng = np.random.default_rng(400 + e0)
+    b = pairs(rng, 1 << 18, e0, e1)
+    q = value(pairs(rng, len(b), f0, f1)).astype(np.float64)
+    x = q * value(b).astype(np.float64)
+    hi = x.astype(np.float32)
+    a = np.stack([hi, (x - hi).astype(np.float32)], axis=1)
+    out = ops(probe, a, b)
+    err = np.abs(value(out[0]) / (value(a) / value(b)) - 1)
+    assert np.isfinite(err).all() and err.max() <= 2.0 ** -44
+    inv = 1 / value(b)
+    err = np.abs(value(out[2]) - inv)
+    assert np.isfinite(err).all() and (err <= 2.0 ** -44 * inv + 2.0 ** -148).all()
