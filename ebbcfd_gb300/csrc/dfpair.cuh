@@ -132,7 +132,10 @@ __device__ __forceinline__ dfp root(dfp a)
     const f2 r = pack2(ebbdf::rsqrt32(x), ebbdf::rsqrt32(y)), h = mul2(pack2(0.5f, 0.5f), r);
     f2 s = mul2(a.hi, r);
     s = fma2(fma2(neg2(s), s, a.hi), h, s);
-    return fast_two_sum2(s, mul2(add2(fma2(neg2(s), s, a.hi), a.lo), h));
+    const f2 t = add2(fma2(neg2(s), s, a.hi), a.lo);
+    f2 c = mul2(t, h);
+    c = fma2(fma2(neg2(c), add2(s, s), t), h, c);
+    return fast_two_sum2(s, c);
 }
 
 }  // namespace ebbdev

@@ -86,7 +86,7 @@ def ops(probe, a, b):
                                        (60, 126, 2.0 ** -44)])
 def test_double_float_roots_over_the_range(probe, e0, e1, tol):
     """Within 2^-44 where the remainder of the FP32 root is an FP32 number, within 2^-22
-    below, singly and in pairs, also beside a zero."""
+    below.  The packed root is the single one's bit for bit, also beside a zero."""
     a = pairs(np.random.default_rng(200 + e0), 1 << 18, e0, e1)
     a[::101] = 0.0
     out = ops(probe, a, pairs(np.random.default_rng(2), len(a), -20, 20))
@@ -96,6 +96,7 @@ def test_double_float_roots_over_the_range(probe, e0, e1, tol):
         assert (r[~pos] == 0.0).all()
         err = np.abs(value(r)[pos] / exact[pos] - 1)
         assert np.isfinite(err).all() and err.max() <= tol
+    assert np.array_equal(out[1].view(np.uint32), out[3].view(np.uint32))
 
 
 @pytest.mark.parametrize("e0,e1,f0,f1", [(-127, -127, 30, 60), (-126, -100, 26, 60), (-20, 20, -20, 20), (100, 126, -60, 0),
