@@ -89,11 +89,15 @@ __device__ __forceinline__ dfp fast_two_sum2(f2 a, f2 b)
     const f2 s = add2(a, b);
     return {s, sub2(b, sub2(s, a))};
 }
+__device__ __forceinline__ dfp two_sum2(f2 a, f2 b)
+{
+    const f2 s = add2(a, b), t = sub2(s, a);
+    return {s, add2(sub2(a, sub2(s, t)), sub2(b, t))};
+}
 __device__ __forceinline__ dfp operator+(dfp a, dfp b)
 {
-    const f2 s = add2(a.hi, b.hi), t = sub2(s, a.hi);
-    const f2 e = add2(sub2(a.hi, sub2(s, t)), sub2(b.hi, t));
-    return fast_two_sum2(s, add2(e, add2(a.lo, b.lo)));
+    const dfp s = two_sum2(a.hi, b.hi);
+    return fast_two_sum2(s.hi, add2(s.lo, add2(a.lo, b.lo)));
 }
 __device__ __forceinline__ dfp operator-(dfp a, dfp b)
 {
@@ -111,18 +115,19 @@ __device__ __forceinline__ dfp half(dfp a)
     const f2 h = pack2(0.5f, 0.5f);
     return {mul2(h, a.hi), mul2(h, a.lo)};
 }
-// 1 / b, as dfloat.h's quotient of 1
-__device__ __forceinline__ dfp recip(dfp b)
+__device__ __forceinline__ dfp operator/(dfp a, dfp b)
 {
     float x, y;
     unpack2(b.hi, x, y);
-    const f2 r0 = pack2(ebbdf::rcp32(x), ebbdf::rcp32(y)), one = pack2(1.0f, 1.0f), nh = neg2(b.hi);
-    const f2 q = fma2(fma2(r0, nh, one), r0, r0);
-    const f2 r = fma2(q, neg2(b.lo), fma2(q, nh, one));
-    f2 l = mul2(r, r0);
-    l = fma2(fma2(l, nh, r), r0, l);
-    return fast_two_sum2(q, l);
+    const f2 r0 = pack2(ebbdf::rcp32(x), ebbdf::rcp32(y)), nh = neg2(b.hi), nl = neg2(b.lo);
+    f2 q = mul2(a.hi, r0);
+    q = fma2(fma2(q, nh, a.hi), r0, q);
+    const dfp r = two_sum2(fma2(q, nh, a.hi), fma2(q, nl, a.lo));
+    const f2 l = mul2(r.hi, r0), left = add2(fma2(l, nl, fma2(l, nh, r.hi)), r.lo);
+    const dfp s = fast_two_sum2(q, l);
+    return fast_two_sum2(s.hi, fma2(left, r0, s.lo));
 }
+__device__ __forceinline__ dfp recip(dfp b) { return both(df(1.0f)) / b; }
 // sqrt of both, which are positive normal numbers (any other element by dfloat.h's sqrt)
 __device__ __forceinline__ dfp root(dfp a)
 {

@@ -66,9 +66,10 @@ __device__ __forceinline__ void roe_flux_df(const df qL[4], const df qR[4], df n
     split(dre, dRho, dRhoE);
     const dfp t = pair(half(qq * qq), -u) * both(dRho) + pair(-sum(vel * dm), sum(dm * n));
     const df G1 = K<df>::gm1 * (first(t) + dRhoE), G2 = second(t);
-    const dfp ra = recip(pair(a, a * a));
-    const df C1 = sum(pair(G1 * second(ra), G2 * first(ra)) * pair(sl, s2));
-    const df C2 = sum(pair(G1 * first(ra), G2) * pair(s2, sl));
+    df ra, G1a2;  // 1 / a and G1 / a^2
+    split(pair(df(1.0f), G1) / pair(a, a * a), ra, G1a2);
+    const df C1 = sum(pair(G1a2, G2 * ra) * pair(sl, s2));
+    const df C2 = sum(pair(G1 * ra, G2) * pair(s2, sl));
     const dfp l = both(l3), c = both(C1);
     dfp D03 = l * dre + pair(C1, C1 * h);
     const dfp D12 = l * dm + c * vel + both(C2) * n;

@@ -123,5 +123,5 @@ def test_quotient_and_root_as_near_as_from_ieee_operations(tmp_path, product):
     out = subprocess.run([build(tmp_path, PRECISION, "precision")] + ["product"] * product, capture_output=True, text=True,
                          check=True).stdout.split()
     q, q0, inv, inv0, s, s0 = [(float(out[k]), float(out[k + 1])) for k in range(0, 12, 2)]
-    for name, now, ieee in (("root", s, s0),):
+    for name, now, ieee in (("quotient", q, q0), ("reciprocal", inv, inv0), ("root", s, s0)):
         assert now[0] <= 1.1 * ieee[0] and now[1] <= ieee[1], (name, now, ieee)

@@ -14,8 +14,9 @@ PROBE = r"""
 #include "dfpair.cuh"
 using namespace ebbdev;
 
-// o = a / b, sqrt(a) singly, and both in pairs of neighbouring elements (n even)
-__global__ void df_ops(int n, const float2 *a, const float2 *b, float2 *div1, float2 *root1, float2 *recip2, float2 *root2)
+// a / b and sqrt(a) singly, and both in pairs of neighbouring elements (n even)
+__global__ void df_ops(int n, const float2 *a, const float2 *b, float2 *div1, float2 *root1, float2 *recip2, float2 *root2,
+                       float2 *div2)
 {
     const int i = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (i + 1 >= n) return;
@@ -29,6 +30,8 @@ __global__ void df_ops(int n, const float2 *a, const float2 *b, float2 *div1, fl
     }
     split(recip(pair(y[0], y[1])), o[0], o[1]);
     for (int k = 0; k < 2; k++) recip2[i + k] = make_float2(o[k].hi, o[k].lo);
+    split(pair(x[0], x[1]) / pair(y[0], y[1]), o[0], o[1]);
+    for (int k = 0; k < 2; k++) div2[i + k] = make_float2(o[k].hi, o[k].lo);
     split(root(pair(x[0], x[1])), o[0], o[1]);
     for (int k = 0; k < 2; k++) root2[i + k] = make_float2(o[k].hi, o[k].lo);
 }
@@ -37,15 +40,15 @@ extern "C" int run_df(int n, const float *a, const float *b, float *out)
 {
     float2 *d = nullptr;
     const size_t s = (size_t)n * sizeof(float2);
-    cudaError_t e = cudaMalloc(&d, 6 * s);
+    cudaError_t e = cudaMalloc(&d, 7 * s);
     if (e == cudaSuccess) e = cudaMemcpy(d, a, s, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(d + n, b, s, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
         df_ops<<<(n / 2 + 127) / 128, 128>>>(n, d, d + n, d + 2 * (size_t)n, d + 3 * (size_t)n, d + 4 * (size_t)n,
-                                             d + 5 * (size_t)n);
+                                             d + 5 * (size_t)n, d + 6 * (size_t)n);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * (size_t)n, 4 * s, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * (size_t)n, 5 * s, cudaMemcpyDeviceToHost);
     cudaFree(d);
     return (int)e;
 }
@@ -76,7 +79,7 @@ def value(p):
 
 
 def ops(probe, a, b):
-    out = np.zeros((4, len(a), 2), dtype=np.float32)
+    out = np.zeros((5, len(a), 2), dtype=np.float32)
     a, b = np.ascontiguousarray(a), np.ascontiguousarray(b)
     assert probe.run_df(len(a), a.ctypes.data, b.ctypes.data, out.ctypes.data) == 0
     return out
@@ -104,8 +107,8 @@ def test_double_float_roots_over_the_range(probe, e0, e1, tol):
 def test_double_float_quotients_over_the_range(probe, e0, e1, f0, f1):
     """Divisors of exponents e0..e1 -- from half the smallest normal number to the largest
     exponent, where a reciprocal or a divisor is subnormal -- and quotients of exponents
-    f0..f1, which keep every remainder an FP32 number: within 2^-44.  Reciprocals in pairs,
-    within that and a unit of the smallest subnormal."""
+    f0..f1, which keep every remainder an FP32 number: within 2^-44, in pairs the same bits.
+    Reciprocals in pairs, within that and a unit of the smallest subnormal."""
     rng = np.random.default_rng(400 + e0)
     b = pairs(rng, 1 << 18, e0, e1)
     q = value(pairs(rng, len(b), f0, f1)).astype(np.float64)
@@ -115,6 +118,7 @@ def test_double_float_quotients_over_the_range(probe, e0, e1, f0, f1):
     out = ops(probe, a, b)
     err = np.abs(value(out[0]) / (value(a) / value(b)) - 1)
     assert np.isfinite(err).all() and err.max() <= 2.0 ** -44
+    assert np.array_equal(out[0].view(np.uint32), out[4].view(np.uint32))
     inv = 1 / value(b)
     err = np.abs(value(out[2]) - inv)
     assert np.isfinite(err).all() and (err <= 2.0 ** -44 * inv + 2.0 ** -148).all()
