@@ -41,6 +41,11 @@
 #else
 #define EBB_SOFT_HD inline
 #endif
+// the host's seeds (a host test puts the device's errors in their place)
+#ifndef EBB_HOST_RCP
+#define EBB_HOST_RCP(x) (1.0f / (x))
+#define EBB_HOST_RSQRT(x) (1.0f / sqrtf(x))
+#endif
 
 namespace ebbsoft {
 
@@ -124,7 +129,7 @@ EBB_SOFT_HD float rcp_seed(float x)
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 #else
-    return 1.0f / x;
+    return EBB_HOST_RCP(x);
 #endif
 }
 EBB_SOFT_HD float rsqrt_seed(float x)
@@ -134,13 +139,14 @@ EBB_SOFT_HD float rsqrt_seed(float x)
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 #else
-    return 1.0f / sqrtf(x);
+    return EBB_HOST_RSQRT(x);
 #endif
 }
-// significand of a seed in (0.5, 1) as an integer of 24 bits (1 taken as 1 - 2^-24)
+// significand of a seed in (0.5, 1) as an integer of 24 bits (1 taken as 1 - 2^-24).  The
+// error of a seed of a value within 2^-24 of 0.5 may take it below: 0.5 is as near.
 EBB_SOFT_HD uint32_t seed_bits(float y)
 {
-    const float c = y < 0.99999994f ? y : 0.99999994f;
+    const float c = fminf(fmaxf(y, 0.5f), 0.99999994f);
     return (as_bits(c) & 0x7fffffu) | 0x800000u;
 }
 
