@@ -14,9 +14,10 @@ using namespace ebbdev;
 
 namespace {
 
-// end of one runIntegrator iteration (app/solver.d:126-249).  blockIdx.y: the instance;
-// blockIdx.x: a part of its rows of block partial sums (step_parts of them, a function of
-// the instance's size alone, so that an instance sums in the same order in any arena).
+// end of one runIntegrator iteration (app/solver.d:126-249).  blockIdx.x: the instance (an
+// arena may have more than the 65,535 that the grid's other dimensions hold); blockIdx.y: a
+// part of its rows of block partial sums (step_parts of them, a function of the instance's
+// size alone, so that an instance sums in the same order in any arena).
 // The block that finishes last adds the parts up in order and runs the epilogue.
 //
 // What bounds it is latency: an FP64 addition takes a warp 64 cycles, so a thread here
@@ -27,7 +28,7 @@ namespace {
 // stages) 101 -> 91 us, of 1M (four stages, 16 parts) 466 -> 450 us, all split precision.
 template <typename T> __global__ void __launch_bounds__(EBB_RED_THREADS) k_step_end(DMesh M, DArrays A, int nblk)
 {
-    const int inst = blockIdx.y, part = blockIdx.x;
+    const int inst = blockIdx.x, part = blockIdx.y;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     DState *st = A.st + inst;
     const int b0 = M.inst_blk ? M.inst_blk[inst] : 0, b1 = M.inst_blk ? M.inst_blk[inst + 1] : nblk;
@@ -240,7 +241,7 @@ int update_grid(const DMesh &M) { return M.n_upd_blocks; }
 int launch_step_end(const DMesh &M, const DArrays &A, int nred_blocks, int precision, void *stream)
 {
     const int n = M.n_inst > 0 ? M.n_inst : 1;
-    const dim3 grid(step_parts(M.max_inst_blocks), n), block(EBB_RED_THREADS);
+    const dim3 grid(n, step_parts(M.max_inst_blocks)), block(EBB_RED_THREADS);
     const cudaStream_t q = (cudaStream_t)stream;
     cudaError_t e;
     if (precision == EBB_PREC_SPLIT)
