@@ -6,9 +6,11 @@ memory latency, so the warps an SM keeps in flight decide their speed; the block
 size and the minimum-blocks argument (a cap on registers per thread -- too low a cap
 spills) set that at compile time.  The FP64 kernels are bound by the FP64 pipe; a few
 more warps can still fill its gaps.  The double-float kernels run long dependent FP32
-sequences with many live values: few warps, and a cap that does not spill.  k_update's block size (256 or 512) is also the
-size of the per-block reduction trees and of the batched arena's update-block map, so
-one value serves all precision forms in a build.
+sequences with many live values: few warps, and a cap that does not spill.  The cell
+kernel of these two forms is k_cell4 (four threads per cell); the shapes of k_cell, which
+takes their first-order and LP-limited solves, are fixed in kernels.cuh.  k_update's block
+size (256 or 512) is also the size of the per-block reductions and of the batched arena's
+update-block map, so one value serves all precision forms in a build.
 
 Every row of candidate settings is one variant of the library (under
 ebbcfd_gb300/_build/tune_<k>/, with -DEBB_* overrides; the variants compile in
@@ -43,17 +45,17 @@ ROOT = os.path.dirname(HERE)
 CANDIDATES = {
     "split": {"cell": [(128, 8), (128, 10), (128, 6), (256, 4), (256, 3), (64, 16), (64, 12)],
               "flux": [(128, 12), (128, 10), (128, 8), (256, 6), (256, 4), (64, 20), (64, 16)],
-              "update": [8, 6, 4, 4, 3, 8, 2]},
-    "fp64": {"cell": [(128, 5), (128, 1), (128, 6), (256, 2), (256, 3), (64, 8), (64, 10)],
-             "flux": [(128, 1), (128, 4), (128, 5), (256, 2), (256, 1), (64, 8), (64, 6)],
+              "update": [8, 6, 4, 4, 3, 3, 2]},
+    "fp64": {"cell": [(128, 8), (128, 6), (128, 10), (256, 4), (256, 3), (64, 16), (64, 12)],
+             "flux": [(128, 1), (128, 4), (128, 5), (256, 2), (128, 6), (64, 8), (64, 6)],
              "update": [3, 1, 2, 2, 1, 4, 1]},
-    "df": {"cell": [(128, 2), (128, 1), (128, 3), (256, 1), (256, 2), (64, 4), (64, 6)],
-           "flux": [(128, 2), (128, 1), (128, 3), (256, 1), (256, 2), (64, 4), (64, 6)],
+    "df": {"cell": [(128, 8), (128, 6), (128, 10), (256, 4), (256, 3), (64, 16), (64, 12)],
+           "flux": [(128, 5), (128, 4), (128, 6), (128, 8), (256, 2), (64, 10), (64, 6)],
            "update": [3, 1, 2, 2, 1, 4, 1]},
     # split precision on inviscid meshes (its own launch-shape profile, timed on the wedge)
     "split_inv": {"cell": [(128, 8), (128, 10), (128, 6), (256, 4), (256, 3), (64, 16), (64, 12)],
                   "flux": [(128, 12), (128, 10), (128, 8), (256, 6), (256, 4), (64, 20), (64, 16)],
-                  "update": [8, 6, 4, 4, 3, 8, 2]},
+                  "update": [8, 6, 4, 4, 3, 5, 2]},
 }
 # the form each candidate set is built and timed in, and on which workload (None: the
 # workload being tuned for)
@@ -61,8 +63,8 @@ FORM = {"split": ("split", None), "fp64": ("fp64", None), "df": ("df", None), "s
 UPD_TB = [256, 256, 256, 512, 512, 256, 512]
 N_ROWS = len(UPD_TB)
 MACRO = {("split", "cell"): ("EBB_CELL_TB_F", "EBB_CELL_MINB_F"), ("split", "flux"): ("EBB_FLUX_TB_F", "EBB_FLUX_MINB_F"),
-         ("fp64", "cell"): ("EBB_CELL_TB_D", "EBB_CELL_MINB_D"), ("fp64", "flux"): ("EBB_FLUX_TB_D", "EBB_FLUX_MINB_D"),
-         ("df", "cell"): ("EBB_CELL_TB_W", "EBB_CELL_MINB_W"), ("df", "flux"): ("EBB_FLUX_TB_W", "EBB_FLUX_MINB_W"),
+         ("fp64", "cell"): ("EBB_CELL4_TB_D", "EBB_CELL4_MINB_D"), ("fp64", "flux"): ("EBB_FLUX_TB_D", "EBB_FLUX_MINB_D"),
+         ("df", "cell"): ("EBB_CELL4_TB_W", "EBB_CELL4_MINB_W"), ("df", "flux"): ("EBB_FLUX_TB_W", "EBB_FLUX_MINB_W"),
          ("split", "update"): ("EBB_UPD_TB", "EBB_UPD_MINB_F"), ("fp64", "update"): ("EBB_UPD_TB", "EBB_UPD_MINB_D"),
          ("df", "update"): ("EBB_UPD_TB", "EBB_UPD_MINB_W"),
          ("split_inv", "cell"): ("EBB_CELL_TB_FI", "EBB_CELL_MINB_FI"),

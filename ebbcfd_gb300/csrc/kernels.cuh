@@ -73,14 +73,8 @@ static_assert(EBB_UPD_TB == 256 || EBB_UPD_TB == 512, "k_update's block reductio
 #ifndef EBB_UPD_MINB_FI
 #define EBB_UPD_MINB_FI 8
 #endif
-#ifndef EBB_CELL_TB_W
-#define EBB_CELL_TB_W 128
-#endif
 #ifndef EBB_FLUX_TB_W
 #define EBB_FLUX_TB_W 128
-#endif
-#ifndef EBB_CELL_MINB_W
-#define EBB_CELL_MINB_W 2
 #endif
 #ifndef EBB_FLUX_MINB_W
 #define EBB_FLUX_MINB_W 2
@@ -88,6 +82,12 @@ static_assert(EBB_UPD_TB == 256 || EBB_UPD_TB == 512, "k_update's block reductio
 #ifndef EBB_UPD_MINB_W
 #define EBB_UPD_MINB_W 3
 #endif
+// k_cell in FP64 and double-float takes first-order and LP-limited solves only (k_cell4 the
+// others): the shapes it was tuned to on the plate while it took every solve
+#define EBB_CELL_TB_D 128
+#define EBB_CELL_MINB_D 6
+#define EBB_CELL_TB_W 256
+#define EBB_CELL_MINB_W 2
 template <typename T, int PR> constexpr int pick(int f, int fi, int d, int w)
 {
     return std::is_same<T, float>::value ? (PR ? fi : f) : (std::is_same<T, double>::value ? d : w);
@@ -113,24 +113,15 @@ template <typename T, int PR> constexpr int upd_minb()
     return pick<T, PR>(EBB_UPD_MINB_F, EBB_UPD_MINB_FI, EBB_UPD_MINB_D, EBB_UPD_MINB_W);
 }
 // k_cell4 (four threads per cell)
-#ifndef EBB_CELL4_TB_D
-#define EBB_CELL4_TB_D 128
-#endif
-#ifndef EBB_CELL4_MINB_D
-#define EBB_CELL4_MINB_D 8
-#endif
-#ifndef EBB_CELL4_TB_W
-#define EBB_CELL4_TB_W 128
-#endif
-#ifndef EBB_CELL4_MINB_W
-#define EBB_CELL4_MINB_W 8
-#endif
 template <typename T> constexpr int cell4_threads() { return is_fp64<T> ? EBB_CELL4_TB_D : EBB_CELL4_TB_W; }
 template <typename T> constexpr int cell4_minb() { return is_fp64<T> ? EBB_CELL4_MINB_D : EBB_CELL4_MINB_W; }
 // an SM holds at most 2048 threads: every (threads, minimum blocks) pair must fit
 static_assert(EBB_CELL_TB_F * EBB_CELL_MINB_F <= 2048 && EBB_CELL_TB_D * EBB_CELL_MINB_D <= 2048 &&
                   EBB_CELL_TB_FI * EBB_CELL_MINB_FI <= 2048,
               "k_cell bounds");
+static_assert(EBB_CELL4_TB_D * EBB_CELL4_MINB_D <= 2048 && EBB_CELL4_TB_W * EBB_CELL4_MINB_W <= 2048 &&
+                  EBB_CELL4_TB_D % 32 == 0 && EBB_CELL4_TB_W % 32 == 0,
+              "k_cell4 bounds");
 static_assert(EBB_FLUX_TB_F * EBB_FLUX_MINB_F <= 2048 && EBB_FLUX_TB_D * EBB_FLUX_MINB_D <= 2048 &&
                   EBB_FLUX_TB_FI * EBB_FLUX_MINB_FI <= 2048,
               "k_flux bounds");
