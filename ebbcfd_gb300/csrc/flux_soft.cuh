@@ -30,25 +30,18 @@
 
 namespace ebbdev {
 
-// S: products on the integer pipe, of the groups below; else on the FP64 pipe (a third of
-// the code: boundary faces).  Products taken on the integer pipe, by group (bit g): the side's own, the convective
-// flux along the normal, the wave decomposition, the viscous matrices and sums
-constexpr int SG_SIDE = 0, SG_CONV = 1, SG_MEAN = 2, SG_WAVE = 3, SG_VMAT = 4, SG_VSUM = 5, SG_OUT = 6, SG_GRAD = 7,
-              SG_LIM = 8, SG_FACE = 9;
-#ifndef EBB_SOFT_GROUPS
-#define EBB_SOFT_GROUPS 0x3ff
-#endif
-template <int GROUP, bool S> __device__ __forceinline__ double sm(double a, double b)
+// S: products on the integer pipe; else on the FP64 pipe (a third of the code: boundary faces)
+template <bool S> __device__ __forceinline__ double sm(double a, double b)
 {
-    if constexpr (S && ((EBB_SOFT_GROUPS >> GROUP) & 1))
+    if constexpr (S)
         return ebbsoft::mul(a, b);
     else
         return a * b;
 }
 // the same for an a that is not zero
-template <int GROUP, bool S> __device__ __forceinline__ double smn(double a, double b)
+template <bool S> __device__ __forceinline__ double smn(double a, double b)
 {
-    if constexpr (S && ((EBB_SOFT_GROUPS >> GROUP) & 1))
+    if constexpr (S)
         return ebbsoft::mul<true>(a, b);
     else
         return a * b;
@@ -68,7 +61,6 @@ struct SoftSide {
 template <bool H, bool S>
 __device__ __forceinline__ void soft_side(const double q[4], double nx, double ny, SoftSide &o, double f[4], bool &bad)
 {
-    constexpr int G = SG_SIDE, C = SG_CONV;
     const double rho = q[0], e = q[3];
     ebbsoft::check<60>(rho, bad);
     bad |= !(ebbsoft::hi_of(rho) < 0x7ff00000u) || ebbsoft::hi_of(rho) == 0u;  // positive
@@ -79,19 +71,19 @@ __device__ __forceinline__ void soft_side(const double q[4], double nx, double n
     const double u = ebbsoft::div(q[1], o.R), v = ebbsoft::div(q[2], o.R);
     o.u = u;
     o.v = v;
-    const double uu = sm<G, S>(u, u), vv = sm<G, S>(v, v);
-    o.rv0 = smn<G, S>(rho, u);
-    o.rv1 = smn<G, S>(rho, v);
-    const double p = smn<G, S>(K<double>::gm1, fma(-0.5, smn<G, S>(rho, uu + vv), e));
+    const double uu = sm<S>(u, u), vv = sm<S>(v, v);
+    o.rv0 = smn<S>(rho, u);
+    o.rv1 = smn<S>(rho, v);
+    const double p = smn<S>(K<double>::gm1, fma(-0.5, smn<S>(rho, uu + vv), e));
     o.p = p;
     const double pe = p + e;
     if (H) o.h = ebbsoft::div(pe, o.R);
-    const double f1 = p + smn<G, S>(rho, uu), f2 = sm<G, S>(o.rv0, v), f3 = sm<G, S>(u, pe);
-    const double h2 = p + smn<G, S>(rho, vv), h3 = sm<G, S>(v, pe);
-    f[0] = sm<C, S>(o.rv0, nx) + sm<C, S>(o.rv1, ny);
-    f[1] = sm<C, S>(f1, nx) + sm<C, S>(f2, ny);
-    f[2] = sm<C, S>(f2, nx) + sm<C, S>(h2, ny);
-    f[3] = sm<C, S>(f3, nx) + sm<C, S>(h3, ny);
+    const double f1 = p + smn<S>(rho, uu), f2 = sm<S>(o.rv0, v), f3 = sm<S>(u, pe);
+    const double h2 = p + smn<S>(rho, vv), h3 = sm<S>(v, pe);
+    f[0] = sm<S>(o.rv0, nx) + sm<S>(o.rv1, ny);
+    f[1] = sm<S>(f1, nx) + sm<S>(f2, ny);
+    f[2] = sm<S>(f2, nx) + sm<S>(h2, ny);
+    f[3] = sm<S>(f3, nx) + sm<S>(h3, ny);
 }
 
 // both sides in one loop: A and B, and the sum of their convective fluxes
@@ -143,18 +135,17 @@ template <bool S>
 __device__ __forceinline__ void roe_flux2_soft(const double qL[4], const double qR[4], double nx, double ny, double out[4],
                                                double &sMax, bool &bad)
 {
-    constexpr int M = SG_MEAN, W = SG_WAVE;
     SoftSide A, B;
     double fs[4];
     soft_sides<true, S>(qL, qR, nx, ny, A, B, fs, bad);
     const double di = ebbsoft::root(ebbsoft::div(B.rho, A.R), bad);
     const double d1 = soft_ratio(1.0, 1.0 + di, bad);
-    const double vel0 = smn<M, S>(d1, smn<M, S>(di, B.u) + A.u);
-    const double vel1 = smn<M, S>(d1, smn<M, S>(di, B.v) + A.v);
-    const double u = sm<M, S>(vel0, nx) + sm<M, S>(vel1, ny);
-    const double h = smn<M, S>(d1, smn<M, S>(di, B.h) + A.h);
-    const double vv = sm<M, S>(vel0, vel0) + sm<M, S>(vel1, vel1);
-    const double a = ebbsoft::root(smn<M, S>(K<double>::gm1d, fma(-0.5, vv, h)), bad);
+    const double vel0 = smn<S>(d1, smn<S>(di, B.u) + A.u);
+    const double vel1 = smn<S>(d1, smn<S>(di, B.v) + A.v);
+    const double u = sm<S>(vel0, nx) + sm<S>(vel1, ny);
+    const double h = smn<S>(d1, smn<S>(di, B.h) + A.h);
+    const double vv = sm<S>(vel0, vel0) + sm<S>(vel1, vel1);
+    const double a = ebbsoft::root(smn<S>(K<double>::gm1d, fma(-0.5, vv, h)), bad);
     bad |= !ebbsoft::divisor_ok(a);
     const double dRV0 = B.rv0 - A.rv0, dRV1 = B.rv1 - A.rv1;
     const double dRho = qR[0] - qL[0], dRhoE = qR[3] - qL[3];
@@ -164,17 +155,17 @@ __device__ __forceinline__ void roe_flux2_soft(const double qL[4], const double 
     // s1 - l3 and twice s2; G1's first term doubled
     const double sl = fma(0.5, l1 + l2, -l3), s2 = l1 - l2;
     const double qq = ebbsoft::root(vv, bad);
-    const double G1 = smn<W, S>(K<double>::gm1, fma(0.5, sm<W, S>(sm<W, S>(qq, qq), dRho), -(sm<W, S>(vel0, dRV0) + sm<W, S>(vel1, dRV1))) + dRhoE);
-    const double G2 = sm<W, S>(-u, dRho) + (sm<W, S>(dRV0, nx) + sm<W, S>(dRV1, ny));
+    const double G1 = smn<S>(K<double>::gm1, fma(0.5, sm<S>(sm<S>(qq, qq), dRho), -(sm<S>(vel0, dRV0) + sm<S>(vel1, dRV1))) + dRhoE);
+    const double G2 = sm<S>(-u, dRho) + (sm<S>(dRV0, nx) + sm<S>(dRV1, ny));
     const ebbsoft::Recip R = ebbsoft::recip(a);
     const double C1 = fma(0.5, ebbsoft::div(G2, R) * s2, soft_ratio(G1, ebbsoft::mul<true>(a, a), bad) * sl);
     const double C2 = fma(0.5, ebbsoft::div(G1, R) * s2, sl * G2);
     ebbsoft::check<400>(C1, bad);
     ebbsoft::check<400>(C2, bad);
-    out[0] = fs[0] - (smn<W, S>(l3, dRho) + C1);
-    out[1] = fs[1] - (smn<W, S>(l3, dRV0) + sm<W, S>(C1, vel0) + sm<W, S>(C2, nx));
-    out[2] = fs[2] - (smn<W, S>(l3, dRV1) + sm<W, S>(C1, vel1) + sm<W, S>(C2, ny));
-    out[3] = fs[3] - (smn<W, S>(l3, dRhoE) + sm<W, S>(C1, h) + sm<W, S>(C2, u));
+    out[0] = fs[0] - (smn<S>(l3, dRho) + C1);
+    out[1] = fs[1] - (smn<S>(l3, dRV0) + sm<S>(C1, vel0) + sm<S>(C2, nx));
+    out[2] = fs[2] - (smn<S>(l3, dRV1) + sm<S>(C1, vel1) + sm<S>(C2, ny));
+    out[3] = fs[3] - (smn<S>(l3, dRhoE) + sm<S>(C1, h) + sm<S>(C2, u));
 }
 
 // twice the Rusanov flux (source/flux.d:66-141, the reduced form of rusanov_flux)
@@ -182,27 +173,26 @@ template <bool S>
 __device__ __forceinline__ void rusanov_flux2_soft(const double qL[4], const double qR[4], double nx, double ny,
                                                    double out[4], double &sMax, bool &bad)
 {
-    constexpr int M = SG_MEAN, W = SG_WAVE;
     SoftSide A, B;
     double fs[4];
     soft_sides<false, S>(qL, qR, nx, ny, A, B, fs, bad);
-    const double rho = ebbsoft::root(smn<M, S>(A.rho, B.rho), bad);
+    const double rho = ebbsoft::root(smn<S>(A.rho, B.rho), bad);
     const double sL = ebbsoft::root(A.rho, bad), sR = ebbsoft::root(B.rho, bad);
     const ebbsoft::Recip D = ebbsoft::recip(sL + sR);
-    const double vel0 = ebbsoft::div(smn<M, S>(sL, A.u) + smn<M, S>(sR, B.u), D);
-    const double vel1 = ebbsoft::div(smn<M, S>(sL, A.v) + smn<M, S>(sR, B.v), D);
-    const double u = sm<M, S>(vel0, nx) + sm<M, S>(vel1, ny);
-    const double p = ebbsoft::div(smn<M, S>(sL, A.p) + smn<M, S>(sR, B.p), D);
-    const double a = ebbsoft::root(smn<M, S>(K<double>::g, ebbsoft::div(p, ebbsoft::recip(rho))), bad);
+    const double vel0 = ebbsoft::div(smn<S>(sL, A.u) + smn<S>(sR, B.u), D);
+    const double vel1 = ebbsoft::div(smn<S>(sL, A.v) + smn<S>(sR, B.v), D);
+    const double u = sm<S>(vel0, nx) + sm<S>(vel1, ny);
+    const double p = ebbsoft::div(smn<S>(sL, A.p) + smn<S>(sR, B.p), D);
+    const double a = ebbsoft::root(smn<S>(K<double>::g, ebbsoft::div(p, ebbsoft::recip(rho))), bad);
     bad |= !ebbsoft::divisor_ok(a);
     double l1, l2, l3;
     soft_speeds(u, a, l1, l2, l3, bad);
     const double s = max4(l1, l2, l3, l3);
     sMax = s;
-    out[0] = fs[0] - smn<W, S>(s, qR[0] - qL[0]);
-    out[1] = fs[1] - smn<W, S>(s, B.rv0 - A.rv0);
-    out[2] = fs[2] - smn<W, S>(s, B.rv1 - A.rv1);
-    out[3] = fs[3] - smn<W, S>(s, qR[3] - qL[3]);
+    out[0] = fs[0] - smn<S>(s, qR[0] - qL[0]);
+    out[1] = fs[1] - smn<S>(s, B.rv0 - A.rv0);
+    out[2] = fs[2] - smn<S>(s, B.rv1 - A.rv1);
+    out[3] = fs[3] - smn<S>(s, qR[3] - qL[3]);
 }
 
 template <bool S>
@@ -224,7 +214,6 @@ template <bool S>
 __device__ __forceinline__ void diffusive_flux2_soft(const ViscConst<double> &vc, double mu, const double q[4],
                                                      const double dq[4][2], double nx, double ny, double out[4], bool &bad)
 {
-    constexpr int M = SG_VMAT, V = SG_VSUM;
     ebbsoft::check<100>(mu, bad);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -236,13 +225,13 @@ __device__ __forceinline__ void diffusive_flux2_soft(const ViscConst<double> &vc
     bad |= (ebbsoft::hi_of(mu) & ebbsoft::kExp) == 0u;
     const double s = ebbsoft::div(ebbsoft::twice(mu), R);
     const double c43 = -4.0 / 3.0, p43 = 4.0 / 3.0, m23 = -2.0 / 3.0, c231 = 2.0 / 3.0 - 1.0;
-    const double uu = sm<M, S>(u, u), vv = sm<M, S>(v, v), gE = smn<M, S>(vc.gP, E);
-    const double b30 = smn<M, S>(s, sm<M, S>(smn<M, S>(c231, u), v));
-    const double sp43 = smn<M, S>(s, p43), sm23 = smn<M, S>(s, m23), sgP = smn<M, S>(s, vc.gP);
-    const double su = smn<M, S>(s, u), sv = smn<M, S>(s, v), tu = smn<M, S>(s, smn<M, S>(m23, u)), tv = smn<M, S>(s, smn<M, S>(m23, v));
+    const double uu = sm<S>(u, u), vv = sm<S>(v, v), gE = smn<S>(vc.gP, E);
+    const double b30 = smn<S>(s, sm<S>(smn<S>(c231, u), v));
+    const double sp43 = smn<S>(s, p43), sm23 = smn<S>(s, m23), sgP = smn<S>(s, vc.gP);
+    const double su = smn<S>(s, u), sv = smn<S>(s, v), tu = smn<S>(s, smn<S>(m23, u)), tv = smn<S>(s, smn<S>(m23, v));
     // row 2 of the x matrices is row 1 of the y ones
-    const double G12 = (zero_plus(sm<V, S>(-sv, dq[0][0])) + smn<V, S>(s, dq[2][0])) +
-                       (zero_plus(sm<V, S>(-su, dq[0][1])) + smn<V, S>(s, dq[1][1]));
+    const double G12 = (zero_plus(sm<S>(-sv, dq[0][0])) + smn<S>(s, dq[2][0])) +
+                       (zero_plus(sm<S>(-su, dq[0][1])) + smn<S>(s, dq[1][1]));
     double Gn[4];  // G0_1, G0_3, G1_2, G1_3
     double z0 = dq[0][0], z1 = dq[1][0], z2 = dq[2][0], z3 = dq[3][0];
     double w0 = dq[0][1], w1 = dq[1][1], w2 = dq[2][1], w3 = dq[3][1];
@@ -264,12 +253,12 @@ __device__ __forceinline__ void diffusive_flux2_soft(const ViscConst<double> &vc
         eB = su;
     };
     auto rows = [&](double &n, double &e) {
-        n = (zero_plus(sm<V, S>(smn<M, S>(s, smn<M, S>(c43, U)), z0)) + smn<V, S>(sp43, zn)) +
-            (zero_plus(sm<V, S>(tV, w0)) + smn<V, S>(sm23, w2));
-        const double t = sm<M, S>(tA, uu) + sm<M, S>(tB, vv) - gE;
-        e = (zero_plus(sm<V, S>(smn<M, S>(s, t), z0)) + sm<V, S>(smn<M, S>(s, sm<M, S>(kA, u)), z1) +
-             sm<V, S>(smn<M, S>(s, sm<M, S>(kB, v)), z2) + smn<V, S>(sgP, z3)) +
-            (zero_plus(sm<V, S>(b30, w0)) + sm<V, S>(eA, w1) + sm<V, S>(eB, w2));
+        n = (zero_plus(sm<S>(smn<S>(s, smn<S>(c43, U)), z0)) + smn<S>(sp43, zn)) +
+            (zero_plus(sm<S>(tV, w0)) + smn<S>(sm23, w2));
+        const double t = sm<S>(tA, uu) + sm<S>(tB, vv) - gE;
+        e = (zero_plus(sm<S>(smn<S>(s, t), z0)) + sm<S>(smn<S>(s, sm<S>(kA, u)), z1) +
+             sm<S>(smn<S>(s, sm<S>(kB, v)), z2) + smn<S>(sgP, z3)) +
+            (zero_plus(sm<S>(b30, w0)) + sm<S>(eA, w1) + sm<S>(eB, w2));
     };
 #pragma unroll 1
     for (int d = 0; d < 2; d++) {
@@ -278,9 +267,9 @@ __device__ __forceinline__ void diffusive_flux2_soft(const ViscConst<double> &vc
         rows(Gn[2], Gn[3]);
         next_direction();
     }
-    out[1] = sm<SG_OUT, S>(Gn[0], nx) + sm<SG_OUT, S>(G12, ny);
-    out[2] = sm<SG_OUT, S>(G12, nx) + sm<SG_OUT, S>(Gn[2], ny);
-    out[3] = sm<SG_OUT, S>(Gn[1], nx) + sm<SG_OUT, S>(Gn[3], ny);
+    out[1] = sm<S>(Gn[0], nx) + sm<S>(G12, ny);
+    out[2] = sm<S>(G12, nx) + sm<S>(Gn[2], ny);
+    out[3] = sm<S>(Gn[1], nx) + sm<S>(Gn[3], ny);
 }
 
 }  // namespace ebbdev

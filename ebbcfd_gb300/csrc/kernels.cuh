@@ -1027,7 +1027,7 @@ __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
                 const long long bits = __double_as_longlong(du);
                 dlo = (unsigned long long)bits > (unsigned long long)dlo ? bits : dlo;
                 dhi = bits > dhi ? bits : dhi;
-                const double px = sm<SG_GRAD, true>(gm.x, du), py = sm<SG_GRAD, true>(gm.y, du);
+                const double px = ebbsoft::mul(gm.x, du), py = ebbsoft::mul(gm.y, du);
                 g0 = j == 0 ? zero_plus(px) : g0 + px;
                 g1 = j == 0 ? zero_plus(py) : g1 + py;
             } else {
@@ -1086,7 +1086,7 @@ __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
         } else if (j >= 0) {
             const typename V2<T>::t nd = ld2<T>(M.g.s_nd, (size_t)j * Cs + i);
             if constexpr (is_fp64<T>) {
-                const double dd = sm<SG_LIM, true>(g0, nd.x) + sm<SG_LIM, true>(g1, nd.y);
+                const double dd = ebbsoft::mul(g0, nd.x) + ebbsoft::mul(g1, nd.y);
                 const double s = soft_ratio(low ? dl : dh, dd, bad);
                 lim = __double2hiint(s) < 0x3ff00000 ? s : 1.0;  // min(1, s), s >= -0
             } else {
@@ -1096,8 +1096,8 @@ __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
     }
     T lg0, lg1;
     if constexpr (is_fp64<T>) {
-        lg0 = sm<SG_LIM, true>(lim, g0);
-        lg1 = sm<SG_LIM, true>(lim, g1);
+        lg0 = ebbsoft::mul(lim, g0);
+        lg1 = ebbsoft::mul(lim, g1);
         ebbsoft::check<400>(lg0, bad);
         ebbsoft::check<400>(lg1, bad);
         if (__any_sync(quad, bad)) {
@@ -1127,7 +1127,7 @@ __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
             const typename V2<T>::t fd = slot(fdk, j);
             T f;
             if constexpr (is_fp64<T>) {
-                f = qi + sm<SG_FACE, true>(lg0, fd.x) + sm<SG_FACE, true>(lg1, fd.y);
+                f = qi + ebbsoft::mul(lg0, fd.x) + ebbsoft::mul(lg1, fd.y);
             } else {
                 df x, y;
                 split(gp * pair(fd.x, fd.y), x, y);
