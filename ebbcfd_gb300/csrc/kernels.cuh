@@ -56,8 +56,9 @@ static_assert(EBB_UPD_TB == 256 || EBB_UPD_TB == 512, "k_update's block reductio
 // Launch shapes per arithmetic type and profile: _F split (float) on viscous meshes
 // (tuned on the Navier-Stokes plate), _FI split on inviscid meshes (tuned on the Euler
 // wedge: no stored gradients, fewer live values), _D plain FP64, _W double-float.  The
-// profile PR (0 viscous or other forms, 1 split inviscid) is a template parameter of the
-// stage kernels because the register cap is a compile-time launch bound.
+// profile PR (0 viscous or other forms, 1 split inviscid, 2 split inviscid on large meshes:
+// shape_profile) is a template parameter of the stage kernels because the register cap is a
+// compile-time launch bound.
 #ifndef EBB_CELL_TB_FI
 #define EBB_CELL_TB_FI 128
 #endif
@@ -110,7 +111,7 @@ template <typename T, int PR> constexpr int flux_minb()
 }
 template <typename T, int PR> constexpr int upd_minb()
 {
-    return pick<T, PR>(EBB_UPD_MINB_F, EBB_UPD_MINB_FI, EBB_UPD_MINB_D, EBB_UPD_MINB_W);
+    return pick<T, PR>(EBB_UPD_MINB_F, PR == 2 ? 8 : EBB_UPD_MINB_FI, EBB_UPD_MINB_D, EBB_UPD_MINB_W);
 }
 // k_cell4 (four threads per cell)
 template <typename T> constexpr int cell4_threads() { return is_fp64<T> ? EBB_CELL4_TB_D : EBB_CELL4_TB_W; }
@@ -1150,7 +1151,8 @@ __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())
 // of the split viscous form (80 of 85): its blocks run in ascending order only (a reversible
 // order spills 40 bytes a thread instead of 16), the test for a stopped solve comes before
 // the gathers, and the geometry takes plain loads; inviscid meshes, with registers to
-// spare, mark it to leave L2 first (500,000 triangles 83.8 against 86.3 us a step).  Measured
+// spare, mark it to leave L2 first (500,000 triangles 83.8 against 86.3 us a step; large ones
+// do not, see shape_profile).  Measured
 // so, per launch and step: 1M plate cells 47.9 -> 39.1 and 424 -> 409 us, 200,000 9.2 -> 8.6
 // and 99.1 -> 98.2 us.
 template <typename T, int MJ, bool LP, bool UNI, int PR>
@@ -1171,11 +1173,11 @@ __global__ void __launch_bounds__(cell_threads<T, PR>(), cell_minb<T, PR>())
         if (M.cell_inst) inst = M.cell_inst[i];
         if constexpr (sizeof(T) == 4) {
             const int Cs = M.Cs;
-            const auto geom = [](const void *p, size_t s) { return PR ? lds2<T>(p, s) : ld2<T>(p, s); };
+            const auto geom = [](const void *p, size_t s) { return PR == 1 ? lds2<T>(p, s) : ld2<T>(p, s); };
 #pragma unroll
             for (int j = 0; j < MJ; j++) {
                 const int *p = M.s_nbr + (size_t)j * Cs + i;
-                pre.nb[j] = PR ? stream(p) : *p;
+                pre.nb[j] = PR == 1 ? stream(p) : *p;
             }
 #pragma unroll
             for (int j = 0; j < MJ; j++) {
@@ -1669,7 +1671,8 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
                                                        int dt_update, int need_dt, int final_stage)
 {
     constexpr bool SPLIT = sizeof(T) == 4;
-    const int blk = ordered_block(M, gridDim.x);
+    constexpr bool LARGE = PR == 2;  // loads where they are used, 32 registers: shape_profile
+    const int blk = LARGE ? (int)blockIdx.x : ordered_block(M, gridDim.x);
     int i, iend, inst = 0;
     if (M.blk_first) {  // batched arena: each block lies inside one instance's cell range
         i = M.blk_first[blk] + threadIdx.x;
@@ -1691,10 +1694,12 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
 #pragma unroll
         for (int j = 0; j < MJ; j++) ev[j] = stream(M.s_edge + (size_t)j * Cs + i);
         ne = UNI ? MJ : M.nedge[i];
-        nia = ld1<T>(M.g.neg_inv_area, i);
-        if (speeds) {
-            perim = ld1<T>(M.g.perim, i);
-            dlen = ld1<T>(M.g.dlen, i);
+        if (!LARGE) {
+            nia = ld1<T>(M.g.neg_inv_area, i);
+            if (speeds) {
+                perim = ld1<T>(M.g.perim, i);
+                dlen = ld1<T>(M.g.dlen, i);
+            }
         }
         if constexpr (SPLIT) {
 #pragma unroll
@@ -1711,7 +1716,7 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
     T *aux = reinterpret_cast<T *>(A.aux);
     T f[MJ][4], fe[MJ], ax[4], qb[4];
     double q0[4];
-    if (act) {
+    auto gather = [&]() {
         const T *fl = reinterpret_cast<const T *>(A.fl);
         const T *fs = reinterpret_cast<const T *>(A.fs);
 #pragma unroll
@@ -1722,7 +1727,8 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
                 fe[j] = speeds ? fs[e] : T(0.0);
             }
         }
-    }
+    };
+    if (!LARGE && act) gather();
     // the solution and the earlier stages, loaded where they are used: held from here on
     // with the flux gathers, they spill (1M plate cells, split: step 450 instead of 433 us)
     auto stage_loads = [&]() {
@@ -1741,6 +1747,7 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
     float fdtc = INFINITY, frm = 0.0f;
     bool bad = false;
     if (act) {
+        if (LARGE) gather();
         // the sums add in edge order
         T r[4] = {T(0.0), T(0.0), T(0.0), T(0.0)};
         T sAve = 0;
@@ -1795,6 +1802,10 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
         }
         T *cdt = reinterpret_cast<T *>(A.cdt);
         if (speeds) {
+            if (LARGE) {
+                perim = ld1<T>(M.g.perim, i);
+                dlen = ld1<T>(M.g.dlen, i);
+            }
             sAve = ratio(sAve, perim);
             T c = ratio(cfl_of<T>(st) * dlen, sAve);
             if (need_dt) {
@@ -1819,9 +1830,11 @@ __global__ void __launch_bounds__(UPD_THREADS, upd_minb<T, PR>()) k_update(DMesh
 #pragma unroll
             for (int k = 0; k < 4; k++) rm = max_abs(rm, r[k]);
         }
-        stage_loads();
+        if (!LARGE) stage_loads();
         T R[4];
+        if (LARGE) nia = ld1<T>(M.g.neg_inv_area, i);
         mul4(r, nia, R);
+        if (LARGE) stage_loads();
         if (P.mms) {
             T S[4];
             ld4(ptr<T>(M.g.src) + 4 * (size_t)i, S);
@@ -2148,20 +2161,29 @@ int launch_update_pr(const DMesh &M, const DPhys &P, const DArrays &A, int stage
     if (grid.x == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = cudaSuccess;
-#define EBB_UPD_MJ(S, MJ)                                                                                         \
-    e = M.uniform ? launch_dep(k_update<T, S, MJ, true, PR>, grid, dim3(UPD_THREADS), s, M, P, A, qin, qout,       \
-                               dt_update, need_dt, final_stage)                                                      \
-                  : launch_dep(k_update<T, S, MJ, false, PR>, grid, dim3(UPD_THREADS), s, M, P, A, qin, qout,      \
-                               dt_update, need_dt, final_stage)
+#define EBB_UPD_U(S, MJ, U)                                                                                        \
+    e = launch_dep(k_update<T, S, MJ, U, PR>, grid, dim3(UPD_THREADS), s, M, P, A, qin, qout, dt_update, need_dt,   \
+                   final_stage)
 #define EBB_UPD(S)                                                                                                 \
     case S:                                                                                                        \
-        if (M.maxJ <= 3)                                                                                           \
-            EBB_UPD_MJ(S, 3);                                                                                      \
-        else if (M.maxJ == 4)                                                                                      \
-            EBB_UPD_MJ(S, 4);                                                                                      \
-        else                                                                                                       \
-            e = launch_dep(k_update<T, S, 6, false, PR>, grid, dim3(UPD_THREADS), s, M, P, A, qin, qout, dt_update,\
-                           need_dt, final_stage);                                                                  \
+        if constexpr (PR == 2) { /* uniform meshes only */                                                         \
+            if (M.maxJ <= 3)                                                                                       \
+                EBB_UPD_U(S, 3, true);                                                                             \
+            else                                                                                                   \
+                EBB_UPD_U(S, 4, true);                                                                             \
+        } else if (M.maxJ <= 3) {                                                                                  \
+            if (M.uniform)                                                                                         \
+                EBB_UPD_U(S, 3, true);                                                                             \
+            else                                                                                                   \
+                EBB_UPD_U(S, 3, false);                                                                            \
+        } else if (M.maxJ == 4) {                                                                                  \
+            if (M.uniform)                                                                                         \
+                EBB_UPD_U(S, 4, true);                                                                             \
+            else                                                                                                   \
+                EBB_UPD_U(S, 4, false);                                                                            \
+        } else {                                                                                                   \
+            EBB_UPD_U(S, 6, false);                                                                                \
+        }                                                                                                          \
         break;
     switch (stage) {
         EBB_UPD(ST_RESID)
@@ -2178,33 +2200,52 @@ int launch_update_pr(const DMesh &M, const DPhys &P, const DArrays &A, int stage
         return -1;
     }
 #undef EBB_UPD
-#undef EBB_UPD_MJ
+#undef EBB_UPD_U
     return ret(e);
 }
 
-// the launch-shape profile: split solves of inviscid meshes take their own shapes
-template <typename T> int shape_profile(const DPhys &P) { return (is_fp32<T> && !P.viscous) ? 1 : 0; }
+// The launch-shape profile: split solves of inviscid meshes take their own shapes, large ones
+// the second of two.  Up to the line a stage's data passes through L2 more than once: the cell
+// kernel marks its geometry to leave it first, and the update kernel has all its loads in
+// flight, at 48 registers and 40 warps per SM.  Beyond it both kernels run at the memory's
+// rate, where evict-first loads and fewer warps lose: plain loads, and on uniform meshes an
+// update kernel that loads each value where it is used, at 32 registers and 64 warps (mixed
+// meshes spill there: 135 against 129 us a launch on 4M cells).  us a step, profile 1 / 2:
+// triangles (RK2) 1M 159 / 163, 2M 294 / 296, 3M 435 / 426, 6M 840 / 827; quads (TVD-RK2) 1M
+// 207.2 / 207.7, 4M 754 / 719, 16M 2928 / 2747; 512 bump channels, 24.3M triangles (TVD-RK2),
+// 3672 / 3508.
+constexpr int kLargeCells = 2500000;
+template <typename T> int shape_profile(const DMesh &M, const DPhys &P)
+{
+    return !is_fp32<T> || P.viscous ? 0 : (M.C < kLargeCells ? 1 : 2);
+}
 
 template <typename T>
 int launch_cell_impl(const DMesh &M, const DPhys &P, const DArrays &A, const T *qin, int limit, void *stream)
 {
-    if constexpr (is_fp32<T>)
-        if (shape_profile<T>(P)) return launch_cell_pr<T, 1>(M, P, A, qin, limit, stream);
+    if constexpr (is_fp32<T>) {
+        const int p = shape_profile<T>(M, P);
+        if (p == 1) return launch_cell_pr<T, 1>(M, P, A, qin, limit, stream);
+        if (p == 2) return launch_cell_pr<T, 2>(M, P, A, qin, limit, stream);
+    }
     return launch_cell_pr<T, 0>(M, P, A, qin, limit, stream);
 }
 template <typename T> int launch_flux_impl(const DMesh &M, const DPhys &P, const DArrays &A, const T *qin, void *stream)
 {
     if constexpr (is_fp32<T>)
-        if (shape_profile<T>(P)) return launch_flux_pr<T, 1>(M, P, A, qin, stream);
+        if (shape_profile<T>(M, P)) return launch_flux_pr<T, 1>(M, P, A, qin, stream);
     return launch_flux_pr<T, 0>(M, P, A, qin, stream);
 }
 template <typename T>
 int launch_update_impl(const DMesh &M, const DPhys &P, const DArrays &A, int stage, const T *qin, T *qout,
                        int dt_update, int need_dt, int final_stage, void *stream)
 {
-    if constexpr (is_fp32<T>)
-        if (shape_profile<T>(P))
-            return launch_update_pr<T, 1>(M, P, A, stage, qin, qout, dt_update, need_dt, final_stage, stream);
+    if constexpr (is_fp32<T>) {
+        const int p = shape_profile<T>(M, P);
+        if (p == 2 && M.uniform && M.maxJ <= 4)
+            return launch_update_pr<T, 2>(M, P, A, stage, qin, qout, dt_update, need_dt, final_stage, stream);
+        if (p) return launch_update_pr<T, 1>(M, P, A, stage, qin, qout, dt_update, need_dt, final_stage, stream);
+    }
     return launch_update_pr<T, 0>(M, P, A, stage, qin, qout, dt_update, need_dt, final_stage, stream);
 }
 
