@@ -39,8 +39,8 @@ template <> struct K<df> {  // the double constants, as double-floats
 // Quotients by one divisor.  FP64: one reciprocal of the divisor serves every quotient,
 // all on the integer pipe (fdiv.h), each the IEEE quotient bit for bit; FP32: plain
 // division, as the split path's flags compile it; double-float: one double-word
-// reciprocal and a double-word product per quotient (relative error a few units of
-// 2^-46, a third of a double-word division's cost).
+// reciprocal (23 operations) and a double-word product (4) per quotient, within a few units
+// of 2^-46.
 template <typename T> struct Div {
     T b;
     __device__ __forceinline__ explicit Div(T d) : b(d) {}

@@ -1,13 +1,18 @@
 // dfpair.cuh -- two double-floats (dfloat.h) side by side in the packed FP32 instructions
 // of sm_100 and later: one instruction adds, multiplies or multiply-adds two FP32 pairs.
 //
-// The double-float flux kernel is bound by issuing and fetching instructions (FMA pipe
+// The double-float flux kernel was bound by issuing and fetching instructions (FMA pipe
 // 46% busy at 53% of the issue slots, a quarter of the time waiting for instructions), so
 // work that comes in twos -- the two sides of a face, the two directions, two components
-// -- takes half the instructions this way.  Every operation is dfloat.h's, step by step.
+// -- takes half the instructions this way.  Now the FMA pipe is 68% busy at 67% of the slots.
 // k_flux, with the shorter quotients and square roots of dfloat.h and the registers this
-// frees (64 a thread, 32 warps per SM instead of 16): 400,000 plate cells 93 -> 65 us,
-// 200,000 triangles (Rusanov) 22 -> 15 us.
+// frees (96 a thread, 20 warps per SM instead of 128 and 16): 400,000 plate cells 93 -> 54
+// us, 200,000 triangles (Rusanov) 22 -> 14 us.
+//
+// Every operation is dfloat.h's, step by step, and gives its bits.  The assembler contracts a
+// packed product whose uses all are sums with them, .rn notwithstanding (seen where a root
+// ended in such a product), so no operation here leaves one: every product is also used in a
+// multiply-add, but for halvings, which are exact.
 #pragma once
 
 #include "dfloat.h"

@@ -5,9 +5,9 @@
 // The plain FP64 flux kernel is bound by the FP64 pipe (a warp instruction every 64
 // cycles of a scheduler: ~440 of them per face kept it 85% busy with 8% of the issue
 // slots used).  Here about 125 remain per face, additions mostly, beside ~6,000 other
-// instructions: the pipe is 67% busy, the integer pipe 54%.  Per launch, 400,000 plate
-// cells: 195 us, 548 us with device_math.cuh; 200,000 triangles (Rusanov): 40 and 136 us
-// (both with the boundary faces' part, which used to run last and alone: k_flux).
+// instructions: the pipe is 72% busy, the integer pipe 57% (1M plate cells).  Per launch,
+// 400,000 plate cells: 195 us, 548 us with device_math.cuh; 200,000 triangles (Rusanov): 40
+// and 136 us (both with the boundary faces' part, which used to run last and alone: k_flux).
 // Three things keep the integer part from costing what it saves:
 //  * code size: as straight-line code a quarter of the warps' time went to instruction
 //    fetches (287 us).  The two sides of a face, the two directions of the viscous

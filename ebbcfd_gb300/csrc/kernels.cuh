@@ -48,8 +48,9 @@ constexpr int ERR_NAN_EDGE = 8, ERR_NAN_CELL = 9, ERR_BC = 11;
 // Threads per block and minimum resident blocks per SM requested through
 // __launch_bounds__ (a register cap per thread: more warps in flight, possibly some
 // spilling).  The FP32 (split) kernels are memory-latency bound and gain from it; the
-// FP64 kernels are FP64-pipe bound.  Values picked by ebbcfd_gb300/autotune.py
-// (per-kernel event timing on GB300; 1 = the compiler's own register choice).
+// FP64 kernels are FP64-pipe bound.  Values and their timings in tuned.h, measured by
+// ebbcfd_gb300/autotune.py (per-kernel event timing on GB300; 1 = the compiler's own
+// register choice).
 #include "tuned.h"
 constexpr int UPD_THREADS = EBB_UPD_TB;
 static_assert(EBB_UPD_TB == 256 || EBB_UPD_TB == 512, "k_update's block reductions take 256 or 512 threads");
@@ -944,7 +945,8 @@ __device__ __forceinline__ bool pressure_negative4(df x, int, unsigned quad)
 // component is formed.  FP64: the products and that quotient run on the integer pipe
 // (softdbl.h) beside the FP64 pipe; the values are cell_body's bit for bit, and a cell with
 // a value out of that arithmetic's range goes to cell_plain.  Bound by the FP64 pipe's
-// additions (61% busy; integer pipe 50%, a sixth of the time fetching instructions).
+// additions and the integer pipe (56% and 56% busy on 1M plate cells, 50% and 61% on 1M
+// triangles; a sixth of the time fetching instructions).
 // Double-float: x and y in packed operations (dfpair.cuh), bound by issue.
 //
 // Lane k loads the geometry of slot k before the wait for the previous kernel: with each
@@ -952,8 +954,8 @@ __device__ __forceinline__ bool pressure_negative4(df x, int, unsigned quad)
 // (double-float) of the warps' time.
 //
 // Measured against one thread per cell, us per launch, FP64 / double-float: 400,000 plate
-// cells 145 (318 all on the FP64 pipe, 143 as here) / 76 (109); 200,000 triangles 54 (155,
-// 52) / 25 (36); 1024 quads, where one warp's latency is the launch's, 7.3 (23, 16) / 5.3
+// cells 147 (318 all on the FP64 pipe, 143 as here) / 80 (109); 200,000 triangles 55 (155,
+// 52) / 25 (36); 1024 quads, where one warp's latency is the launch's, 7.3 (23, 16) / 5.1
 // (14).
 template <typename T, int MJ, bool UNI>
 __global__ void __launch_bounds__(cell4_threads<T>(), cell4_minb<T>())

@@ -320,7 +320,7 @@ typedef struct ebb_server_options {
                               step limit or tEnd (default 1) */
     int32_t stall_steps;   /* default 1000 */
     int32_t finish_precision; /* form of that continuation: EBB_PREC_FP64 (default) or
-                                 EBB_PREC_DF (double-float: about 3.7x FP64's speed on the
+                                 EBB_PREC_DF (double-float: about 3.6x FP64's speed on the
                                  4.0M-cell viscous plate, within ~1e-10 of its forces) */
 } ebb_server_options;
 

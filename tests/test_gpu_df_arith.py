@@ -16,7 +16,7 @@ using namespace ebbdev;
 
 // a / b and sqrt(a) singly, and both in pairs of neighbouring elements (n even)
 __global__ void df_ops(int n, const float2 *a, const float2 *b, float2 *div1, float2 *root1, float2 *recip2, float2 *root2,
-                       float2 *div2)
+                       float2 *div2, float2 *sums1, float2 *sums2)
 {
     const int i = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (i + 1 >= n) return;
@@ -32,6 +32,14 @@ __global__ void df_ops(int n, const float2 *a, const float2 *b, float2 *div1, fl
     for (int k = 0; k < 2; k++) recip2[i + k] = make_float2(o[k].hi, o[k].lo);
     split(pair(x[0], x[1]) / pair(y[0], y[1]), o[0], o[1]);
     for (int k = 0; k < 2; k++) div2[i + k] = make_float2(o[k].hi, o[k].lo);
+    // products under sums and differences, of like and unlike sign
+    const dfp X = pair(x[0], x[1]), Y = pair(y[0], y[1]);
+    split((X * Y + X) * Y - (X * X - Y * Y), o[0], o[1]);
+    for (int k = 0; k < 2; k++) {
+        const df s = (x[k] * y[k] + x[k]) * y[k] - (x[k] * x[k] - y[k] * y[k]);
+        sums1[i + k] = make_float2(s.hi, s.lo);
+        sums2[i + k] = make_float2(o[k].hi, o[k].lo);
+    }
     split(root(pair(x[0], x[1])), o[0], o[1]);
     for (int k = 0; k < 2; k++) root2[i + k] = make_float2(o[k].hi, o[k].lo);
 }
@@ -40,15 +48,15 @@ extern "C" int run_df(int n, const float *a, const float *b, float *out)
 {
     float2 *d = nullptr;
     const size_t s = (size_t)n * sizeof(float2);
-    cudaError_t e = cudaMalloc(&d, 7 * s);
+    cudaError_t e = cudaMalloc(&d, 9 * s);
     if (e == cudaSuccess) e = cudaMemcpy(d, a, s, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(d + n, b, s, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
         df_ops<<<(n / 2 + 127) / 128, 128>>>(n, d, d + n, d + 2 * (size_t)n, d + 3 * (size_t)n, d + 4 * (size_t)n,
-                                             d + 5 * (size_t)n, d + 6 * (size_t)n);
+                                             d + 5 * (size_t)n, d + 6 * (size_t)n, d + 7 * (size_t)n, d + 8 * (size_t)n);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * (size_t)n, 5 * s, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * (size_t)n, 7 * s, cudaMemcpyDeviceToHost);
     cudaFree(d);
     return (int)e;
 }
@@ -79,7 +87,7 @@ def value(p):
 
 
 def ops(probe, a, b):
-    out = np.zeros((5, len(a), 2), dtype=np.float32)
+    out = np.zeros((7, len(a), 2), dtype=np.float32)
     a, b = np.ascontiguousarray(a), np.ascontiguousarray(b)
     assert probe.run_df(len(a), a.ctypes.data, b.ctypes.data, out.ctypes.data) == 0
     return out
@@ -122,3 +130,10 @@ def test_double_float_quotients_over_the_range(probe, e0, e1, f0, f1):
     inv = 1 / value(b)
     err = np.abs(value(out[2]) - inv)
     assert np.isfinite(err).all() and (err <= 2.0 ** -44 * inv + 2.0 ** -148).all()
+
+
+def test_packed_sums_of_products_are_the_single_ones(probe):
+    """Bit for bit: a product contracted with the sum that takes it would not be."""
+    rng = np.random.default_rng(6)
+    out = ops(probe, pairs(rng, 1 << 18, -3, 3), -pairs(rng, 1 << 18, -3, 3))
+    assert np.array_equal(out[5].view(np.uint32), out[6].view(np.uint32))
